@@ -96,6 +96,9 @@ static Layout make_layout(int n, int D, int lpd, int prec) {
   y.scale32 = take(prec == PGJ_FP32 ? sizeof(float) * N3 * D : 0);
   // boundary rows of the halo-free FP32 operator: n planes x n / ty tiles x 3n per load, ty >= 2
   y.qb = take(prec == PGJ_FP32 && n == 64 ? sizeof(float) * (N3 / 2 + 3 * size_t(n)) * L : 0);
+  const size_t halo = resident_halo_bytes(n, prec);
+  y.scale_pl = take(halo && prec == PGJ_FP64 ? sizeof(double) * N3 * D : 0);
+  y.halo = take(halo * L);
   y.total = o;
   return y;
 }
@@ -286,7 +289,9 @@ static int capture_pcg(pgj_ctx* c, int L, cudaStream_t s, bool reliable = false)
 // true-residual replacements, fold, certify; mixed sweeps -> one refinement sweep.
 static int capture_attempt(pgj_ctx* c, int L, cudaStream_t s) {
   int st;
-  if (c->prec == PGJ_FP32 && c->mixed_mode == 0) {
+  if (uses_resident(c)) {
+    st = launch_resident(c, L, s);
+  } else if (c->prec == PGJ_FP32 && c->mixed_mode == 0) {
     st = launch_rel_start(c, L, s);
     if (!st) {
       c->scal = c->scal_in;
@@ -461,6 +466,9 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
     c->hf = c->qb != nullptr && !(e && e[0] == '0') ? 1 : 0;
   }
   c->shat = b + y.shat;
+  c->scale_pl = reinterpret_cast<double*>(b + y.scale_pl);
+  c->halo = b + y.halo;
+  c->res = resident_prepare(n, precision);
   c->scale32 = precision == PGJ_FP32 ? reinterpret_cast<float*>(b + y.scale32) : nullptr;
   c->partials = reinterpret_cast<double*>(b + y.partials);
   c->scal_out = reinterpret_cast<LoadScalars*>(b + y.scal);
@@ -691,7 +699,9 @@ int pgj_solve_wait(pgj_ctx* c, pgj_load_info* info, void* stream) {
   // 7, with the FP32 scale copy) after the mask / recurrence-start kernel
   const long long body = (c->fused ? 4 : 8) + (c->prec == PGJ_FP32 ? 1 : 0);
   const long long first = first_direction_launches(c);
-  if (c->prec == PGJ_FP32)  // rel start, first direction, fold, certify, decide; 3 per replacement
+  if (uses_resident(c))  // scale copy, the resident recurrence, certify, decide
+    c->last_launches = 2 + 3 + attempts * (2 + 3 + 1);
+  else if (c->prec == PGJ_FP32)  // rel start, first direction, fold, certify, decide; 3 per replacement
     c->last_launches = 2 + 3 + attempts * (1 + first + 1 + 3 + 1) + body * cnt[5] + 3LL * cnt[3];
   else  // init mask, first direction, certify, decide
     c->last_launches = 2 + 3 + attempts * (1 + first + 3 + 1) + body * cnt[5];

@@ -73,10 +73,11 @@ constexpr int kAuxDoubles = kAuxPartials + kMaxPartials;
 
 struct Layout {
   size_t a, scale, scale32, symbol, symbol32, tw, solutions, f, x, r, p, q, sw, spec, shat, partials, scal, macros,
-      cond, r64, d, aux, qb, total;
+      cond, r64, d, aux, qb, scale_pl, halo, total;
 };
 
 struct Graphs;
+struct ResidentKernel;
 
 }  // namespace pgj
 
@@ -113,6 +114,9 @@ struct pgj_ctx {
   void* sw;            // (L, 3N) T  s . w (unprojected preconditioned residual)
   void* spec;          // (L, 3, n, n, nsp) complex T
   void* shat;          // (D, 3, n, n, nsp) complex T: DFT of each component of the scale field
+  double* scale_pl;    // FP64 contexts with a cluster-resident PCG: (D, 3, N) copy of scale by component
+  char* halo;          // per load, the planes its cluster's blocks hand to each other
+  const pgj::ResidentKernel* res;  // cluster-resident PCG of this grid and precision, or null
   int fused;           // PCG iteration as operator + slab-fused update/transform kernels
   double* partials;    // (L, kPartialQ * kMaxPartials)
   pgj::LoadScalars* scal;  // L records used by the kernels being launched (outer or inner)
@@ -187,6 +191,15 @@ int prepare_slab_kernels();
 int launch_fxy(pgj_ctx* c, int loads, int prec, int mode, void* u, cudaStream_t s);
 int launch_ifxy(pgj_ctx* c, int loads, int prec, bool init, cudaStream_t s, cudaGraphConditionalHandle h,
                 bool set_cond);
+// cluster-resident PCG (pgj_resident.cu): a whole attempt's recurrence in one launch
+const ResidentKernel* resident_prepare(int n, int prec);
+size_t resident_halo_bytes(int n, int prec);
+int launch_resident(pgj_ctx* c, int loads, cudaStream_t s);
+// The resident kernel runs the plain recurrences: the flexible direction update, FP64 arithmetic on FP32
+// vectors and the refinement sweeps keep the separate kernels, as does a context set to step-by-step.
+inline bool uses_resident(const pgj_ctx* c) {
+  return c->res && c->fused && !c->flex && !c->op64 && !(c->prec == PGJ_FP32 && c->mixed_mode == 1);
+}
 // pcg (pgj_pcg.cu)
 int launch_update_ur(pgj_ctx* c, int loads, int prec, double* u64, void* uT, cudaStream_t s);
 int launch_update_p(pgj_ctx* c, int loads, int prec, bool init, cudaStream_t s, cudaGraphConditionalHandle h,

@@ -1,0 +1,134 @@
+// Host side of the cluster-resident PCG (pgj_resident.cuh): the table of built shapes, whether the
+// device can co-schedule a grid's clusters, and the launch.
+#include "pgj_resident.cuh"
+#include <cstdlib>
+#include <map>
+#include <mutex>
+#include <utility>
+
+namespace pgj {
+
+void resident_f64a(ResidentKernel* out, int* count);
+void resident_f64b(ResidentKernel* out, int* count);
+void resident_f32a(ResidentKernel* out, int* count);
+void resident_f32b(ResidentKernel* out, int* count);
+
+namespace {
+constexpr int kMaxResident = 64;
+struct Table {
+  ResidentKernel k[kMaxResident];
+  int count = 0;
+  Table() {
+    resident_f64a(k, &count);
+    resident_f64b(k, &count);
+    resident_f32a(k, &count);
+    resident_f32b(k, &count);
+  }
+};
+const Table& table() {
+  static const Table t;
+  return t;
+}
+
+cudaLaunchConfig_t config(const ResidentKernel& k, int loads, cudaLaunchAttribute* at, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(k.cl * loads));
+  cfg.blockDim = dim3(unsigned(k.nt));
+  cfg.dynamicSmemBytes = k.smem;
+  cfg.stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = unsigned(k.cl);
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+std::mutex g_mutex;
+std::map<std::pair<const void*, int>, bool> g_fits;  // per kernel and device
+}  // namespace
+
+const ResidentKernel* resident_find(int n, int prec) {
+  const Table& t = table();
+  for (int i = 0; i < t.count; ++i)
+    if (t.k[i].n == n && t.k[i].prec == prec) return &t.k[i];
+  return nullptr;
+}
+
+size_t resident_halo_bytes(int n, int prec) {
+  const ResidentKernel* k = resident_find(n, prec);
+  return k ? k->halo : 0;
+}
+
+// Sets the kernel's launch limits on the current device and asks whether one cluster can be resident
+// there at all (a device partition may have too few SMs in a cluster's reach).
+const ResidentKernel* resident_prepare(int n, int prec) {
+  const char* e = std::getenv("PGJ_RESIDENT");
+  if (e && e[0] == '0') return nullptr;
+  const ResidentKernel* k = resident_find(n, prec);
+  int device = 0;
+  if (!k || cudaGetDevice(&device) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lock(g_mutex);
+  const auto key = std::make_pair(k->fn, device);
+  auto it = g_fits.find(key);
+  if (it == g_fits.end()) {
+    cudaError_t err = cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
+    if (err == cudaSuccess && k->cl > 8)
+      err = cudaFuncSetAttribute(k->fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    int clusters = 0;
+    if (err == cudaSuccess) {
+      cudaLaunchAttribute at;
+      const cudaLaunchConfig_t cfg = config(*k, 1, &at, nullptr);
+      err = cudaOccupancyMaxActiveClusters(&clusters, k->fn, &cfg);
+    }
+    if (err != cudaSuccess) cudaGetLastError();  // not launchable here: the separate kernels serve
+    it = g_fits.emplace(key, err == cudaSuccess && clusters >= 1).first;
+  }
+  return it->second ? k : nullptr;
+}
+
+// out[c][node] = T(s[3 node + c]) for every design
+template <typename T>
+__global__ void k_scale_planes(size_t N, const double* __restrict__ s, T* __restrict__ out) {
+  s += size_t(blockIdx.y) * 3 * N;
+  out += size_t(blockIdx.y) * 3 * N;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x) {
+    const double a = s[3 * i], b = s[3 * i + 1], c = s[3 * i + 2];
+    out[i] = T(a);
+    out[N + i] = T(b);
+    out[2 * N + i] = T(c);
+  }
+}
+
+int launch_resident(pgj_ctx* c, int loads, cudaStream_t s) {
+  const ResidentKernel& k = *c->res;
+  const bool f32 = c->prec == PGJ_FP32;
+  const size_t N = size_t(c->N);
+  const dim3 grid(unsigned((N + 255) / 256 < 148 ? (N + 255) / 256 : 148), unsigned((loads + c->lpd - 1) / c->lpd));
+  if (f32) k_scale_planes<float><<<grid, 256, 0, s>>>(N, c->scale, c->scale32);
+  else k_scale_planes<double><<<grid, 256, 0, s>>>(N, c->scale, c->scale_pl);
+  int st = check_launch();
+  if (st) return st;
+  ResidentArgs A;
+  A.lpd = c->lpd; A.cap = c->cap; A.loads = loads;
+  A.a = c->a;
+  A.f = c->f; A.x = c->x;
+  A.q = c->q; A.spec = c->spec; A.q64 = c->r64;
+  A.halo = c->halo; A.out = c->scal_out; A.counters = c->cond; A.rel_delta2 = c->rel_delta2; A.kc = c->kc;
+  if (f32) {
+    A.sp = c->scale32; A.sym = c->symbol32; A.tw = static_cast<double2*>(c->tw) + c->n;
+    A.r0 = c->r64; A.r = c->r; A.d = c->d; A.p = c->p;
+  } else {
+    // the certified residual's buffer becomes the correction, p and s.w buffers hold r and p
+    A.sp = c->scale_pl; A.sym = c->symbol; A.tw = c->tw;
+    A.r0 = static_cast<const double*>(c->r); A.r = c->p; A.d = c->r; A.p = c->sw;
+  }
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = config(k, loads, &at, s);
+  void* args[] = {&A};
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, k.fn, args);
+  return e == cudaSuccess ? PGJ_OK : set_cuda_error(e);
+}
+
+}  // namespace pgj
