@@ -184,16 +184,19 @@ long long pgj_last_launches(pgj_ctx* ctx);
  * back-to-back launches of that kernel (after two warm launches; the values drift, the work does
  * not). Writes PGJ_PROFILE_KERNELS mean durations (ms) and algorithmic bytes per launch
  * (HOST arrays) in the order: operator, update_ur, fft_x, fft_y, fft_z+symbol, ifft_y, ifft_x,
- * update_p. Leaves the context's iterate undefined (the next pgj_solve starts from its u). */
+ * update_p; the four-kernel iteration fills the first four (operator, update + transforms, z pass, inverse
+ * + direction) and leaves zeros. Leaves the context's iterate undefined (the next pgj_solve starts from its u). */
 #define PGJ_PROFILE_KERNELS 8
 int pgj_profile_iteration(pgj_ctx* ctx, int loads, const double* macros, int reps, double* ms, double* bytes,
                           void* stream);
 
 /* Kernel set of the PCG iteration (no reference counterpart; both give the reference's recurrence).
  * 1: four kernels per iteration (operator; update + x/y transforms; z pass; inverse x/y + direction
- * update), used when a transform slab fits in shared memory; 0: the operator, the two vector updates
- * and the five Green passes as separate kernels. pgj_set_fused_iteration returns
- * PGJ_ERR_UNSUPPORTED for 1 when the slab does not fit. */
+ * update), or on small grids one resident kernel for all of them; 0: the operator, the two vector
+ * updates and the five Green passes as separate kernels. 1 is the default where two transform planes fit
+ * in an SM's shared memory (n <= 80 in FP64, 108 in FP32); pgj_set_fused_iteration returns
+ * PGJ_ERR_UNSUPPORTED for 1 on other grids. Those report 0, and the library runs the four-kernel form
+ * there too as long as one plane pair fits (n <= 108 in FP64, 128 in FP32), unless 0 is set explicitly. */
 int pgj_fused_iteration(pgj_ctx* ctx);
 int pgj_set_fused_iteration(pgj_ctx* ctx, int on);
 

@@ -169,6 +169,7 @@ struct LoadScalars {
   int frozen;       // batched contexts: this load's design took its last attempt (later attempts skip it)
   int restarts;     // restarts taken by this load's design
   double rz_cross;  // flexible beta: new residual . previous preconditioned residual
+  int step;         // plane kernels: a step alpha p of the correction is pending (taken with the next direction)
   int ticket[8];    // per-kernel block tickets for the last-block finalizers
 };
 

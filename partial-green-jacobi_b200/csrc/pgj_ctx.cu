@@ -43,20 +43,15 @@ struct Graphs {
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-DesignScope::DesignScope(pgj_ctx* ctx, int d) : c(ctx), a(ctx->a), scale(ctx->scale), scale32(ctx->scale32), shat(ctx->shat) {
-  const size_t N = size_t(c->N), nsp = size_t(c->ns + (c->ns & 1));
-  const size_t tsz = c->prec == PGJ_FP32 ? 4 : 8;
+DesignScope::DesignScope(pgj_ctx* ctx, int d) : c(ctx), a(ctx->a), scale(ctx->scale) {
+  const size_t N = size_t(c->N);
   c->a = a + d * N;
   c->scale = scale + d * 3 * N;
-  if (scale32) c->scale32 = scale32 + d * 3 * N;
-  c->shat = static_cast<char*>(shat) + d * 2 * tsz * 3 * size_t(c->n) * c->n * nsp;
 }
 
 DesignScope::~DesignScope() {
   c->a = a;
   c->scale = scale;
-  c->scale32 = scale32;
-  c->shat = shat;
 }
 
 // D designs of `lpd` loads each: per-design fields (a, scale, scale32, shat) are D blocks, per-load
@@ -74,8 +69,7 @@ static Layout make_layout(int n, int D, int lpd, int prec) {
   y.macros = take(sizeof(double) * 6 * size_t(L));
   y.cond = take(64);
   y.aux = take(sizeof(double) * kAuxDoubles);
-  // twiddles (double2[n], float2[n]) and the per-axis Green factors (float4[n]: m, v, d)
-  y.tw = take(size_t(n) * (sizeof(double2) + sizeof(float2) + sizeof(float4)));
+  y.tw = take(size_t(n) * (sizeof(double2) + sizeof(float2)));  // twiddles
   const size_t pslots = size_t(kPartialQ * L > 24 ? kPartialQ * L : 24);
   y.partials = take(sizeof(double) * pslots * kMaxPartials);
   y.a = take(sizeof(double) * N * D);
@@ -86,7 +80,7 @@ static Layout make_layout(int n, int D, int lpd, int prec) {
   y.f = take(sizeof(double) * N3 * L);
   y.x = take(sizeof(double) * N3 * L);
   y.r64 = take(prec == PGJ_FP32 ? sizeof(double) * N3 * L : 0);
-  y.d = take(prec == PGJ_FP32 ? tsz * N3 * L : 0);
+  y.d = take(prec == PGJ_FP32 || planes_find(n, prec) ? tsz * N3 * L : 0);
   y.r = take(tsz * N3 * L);
   y.p = take(tsz * N3 * L);
   y.q = take(tsz * N3 * L);
@@ -97,7 +91,7 @@ static Layout make_layout(int n, int D, int lpd, int prec) {
   // boundary rows of the halo-free FP32 operator: n planes x n / ty tiles x 3n per load, ty >= 2
   y.qb = take(prec == PGJ_FP32 && n == 64 ? sizeof(float) * (N3 / 2 + 3 * size_t(n)) * L : 0);
   const size_t halo = resident_halo_bytes(n, prec);
-  y.scale_pl = take(halo && prec == PGJ_FP64 ? sizeof(double) * N3 * D : 0);
+  y.scale_pl = take(prec == PGJ_FP64 && planes_find(n, prec) ? sizeof(double) * N3 * D : 0);
   y.halo = take(halo * L);
   y.total = o;
   return y;
@@ -121,11 +115,11 @@ static int capture_iteration(pgj_ctx* c, int L, cudaStream_t s, cudaGraphConditi
   const int prec = c->prec;
   int st;
   if ((st = launch_recurrence_operator(c, L, prec, s))) return st;
-  if (c->fused) {
-    // u += alpha p, r -= alpha q and the x/y transforms of s.r; z pass; inverse x/y and p update
-    if ((st = launch_fxy(c, L, prec, kSlabUpdateL, prec == PGJ_FP32 ? c->d : static_cast<void*>(c->x), s))) return st;
-    if ((st = launch_fz_fused(c, L, prec, false, s))) return st;
-    return launch_ifxy(c, L, prec, false, s, h, last);
+  if (c->four) {
+    // r -= alpha q and the x/y transforms of s.r; z pass; inverse x/y, d += alpha p and the next p
+    if ((st = launch_planes_fwd(c, L, kPlanesUpdate, s))) return st;
+    if ((st = launch_planes_z(c, L, false, s))) return st;
+    return launch_planes_inv(c, L, false, s, h, last);
   }
   if (prec == PGJ_FP32) st = launch_update_ur(c, L, prec, nullptr, c->d, s);
   else st = launch_update_ur(c, L, prec, c->x, nullptr, s);
@@ -134,24 +128,18 @@ static int capture_iteration(pgj_ctx* c, int L, cudaStream_t s, cudaGraphConditi
   return launch_update_p(c, L, prec, false, s, h, last);
 }
 
-// First direction p = M r of a recurrence (the masks are set): unfused Green + p = z, or the fused
-// form, which first refreshes DFT(s) in case the scale field was rewritten through its view.
-static long long first_direction_launches(const pgj_ctx* c) {
-  // per design DFT(s) (3) [+ FP32 scale], then 3; or Green (5) + p
-  return c->fused ? (long long)c->D * (c->prec == PGJ_FP32 ? 4 : 3) + 3 : 6;
-}
+// First direction p = M r of a recurrence (the masks are set): the Green passes and p = z, or the plane
+// kernels, which first refresh the scale copies and DFT(s) in case the scale was rewritten through its view.
+static long long first_direction_launches(const pgj_ctx* c) { return c->four ? 3 + 3 : 6; }
 
 static int capture_first_direction(pgj_ctx* c, int L, cudaStream_t s) {
   int st;
-  if (c->fused) {
-    for (int d = 0; d < c->D; ++d) {
-      DesignScope view(c, d);
-      if ((st = build_shat(c, s))) return st;
-      if (c->prec == PGJ_FP32 && (st = launch_scale32(c, s))) return st;
-    }
-    if ((st = launch_fxy(c, L, c->prec, kSlabInitL, nullptr, s))) return st;
-    if ((st = launch_fz_fused(c, L, c->prec, true, s))) return st;
-    return launch_ifxy(c, L, c->prec, true, s, 0, false);
+  if (c->four) {
+    if ((st = launch_scale_planes(c, L, s))) return st;
+    if ((st = launch_planes_shat(c, L, s))) return st;
+    if ((st = launch_planes_fwd(c, L, kPlanesInit, s))) return st;
+    if ((st = launch_planes_z(c, L, true, s))) return st;
+    return launch_planes_inv(c, L, true, s, 0, false);
   }
   st = launch_green(c, L, c->prec, c->r, true, s);
   return st ? st : launch_update_p(c, L, c->prec, true, s, 0, false);
@@ -212,14 +200,15 @@ static int capture_into(cudaGraph_t body, F&& fn) {
 // operator, update, IF(any load flagged){x += d; r64 = f - K64 x; r = T(r64)}, Green, p update.
 static int capture_iteration_rel(pgj_ctx* c, int L, cudaStream_t s, cudaGraphConditionalHandle hw) {
   int st;
-  const bool fused = c->fused != 0;
+  const bool fused = c->four != 0;
   if ((st = launch_recurrence_operator(c, L, PGJ_FP32, s))) return st;
-  if (fused) st = launch_fxy(c, L, PGJ_FP32, kSlabUpdateL, c->d, s);
-  else st = launch_update_ur(c, L, PGJ_FP32, nullptr, c->d, s);
-  if (st) return st;
   cudaGraphConditionalHandle hif = 0;
   if ((st = make_handle(s, &hif, 0))) return st;
-  if ((st = launch_rel_cond(c, L, hif, s))) return st;
+  // the plane kernels set the IF condition themselves (update: a load was flagged; sync: taken)
+  if (fused) st = launch_planes_fwd(c, L, kPlanesUpdate, s, hif);
+  else st = launch_update_ur(c, L, PGJ_FP32, nullptr, c->d, s);
+  if (st) return st;
+  if (!fused && (st = launch_rel_cond(c, L, hif, s))) return st;
   cudaGraph_t ifbody = nullptr;
   if ((st = add_conditional(s, &hif, 0, cudaGraphCondTypeIf, &ifbody))) return st;
   st = capture_into(ifbody, [&](cudaStream_t s3) {
@@ -231,12 +220,12 @@ static int capture_iteration_rel(pgj_ctx* c, int L, cudaStream_t s, cudaGraphCon
     c->scal = saved;
     if (r) return r;
     // flagged loads restart from T(r64); the fused form also re-transforms their residual
-    return fused ? launch_fxy(c, L, PGJ_FP32, kSlabSyncL, nullptr, s3) : launch_rel_sync(c, L, s3);
+    return fused ? launch_planes_fwd(c, L, kPlanesSync, s3, hif) : launch_rel_sync(c, L, s3);
   });
   if (st) return st;
   if (fused) {
-    if ((st = launch_fz_fused(c, L, PGJ_FP32, false, s))) return st;
-    return launch_ifxy(c, L, PGJ_FP32, false, s, hw, true);
+    if ((st = launch_planes_z(c, L, false, s))) return st;
+    return launch_planes_inv(c, L, false, s, hw, true);
   }
   if ((st = launch_green(c, L, PGJ_FP32, c->r, false, s))) return st;
   return launch_update_p(c, L, PGJ_FP32, false, s, hw, true);
@@ -309,7 +298,12 @@ static int capture_attempt(pgj_ctx* c, int L, cudaStream_t s) {
     if (!st) st = launch_inner_finish(c, L, s);
   } else {
     st = launch_init_mask(c, L, s);
+    if (!st && c->four) {
+      const cudaError_t e = cudaMemsetAsync(c->d, 0, sizeof(double) * 3 * size_t(c->N) * L, s);
+      if (e != cudaSuccess) st = set_cuda_error(e);
+    }
     if (!st) st = capture_pcg(c, L, s);
+    if (!st && c->four) st = launch_fold64(c, L, s);
   }
   if (!st) st = capture_cert(c, L, s);
   return st;
@@ -459,9 +453,6 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
   c->qb = precision == PGJ_FP32 && n == 64 ? static_cast<void*>(b + y.qb) : nullptr;
   c->hg = hf_geom(n, loads);
   {
-    // the halo-free operator pays off where the slab update's first-row pass is cheap: the n = 64
-    // register-transform path (row tests by shifts); measured per size, every other grid was slower
-    // per iteration with it (n = 16: 51.7 vs 47.6 us, 54: 263 vs 247, 96: 687 vs 683)
     const char* e = std::getenv("PGJ_HF");
     c->hf = c->qb != nullptr && !(e && e[0] == '0') ? 1 : 0;
   }
@@ -469,12 +460,13 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
   c->scale_pl = reinterpret_cast<double*>(b + y.scale_pl);
   c->halo = b + y.halo;
   c->res = resident_prepare(n, precision);
+  c->planes = planes_find(n, precision);
   c->scale32 = precision == PGJ_FP32 ? reinterpret_cast<float*>(b + y.scale32) : nullptr;
   c->partials = reinterpret_cast<double*>(b + y.partials);
   c->scal_out = reinterpret_cast<LoadScalars*>(b + y.scal);
   c->scal_in = c->scal_out + c->L;
   c->scal = c->scal_out;
-  c->d = precision == PGJ_FP32 ? static_cast<void*>(b + y.d) : nullptr;
+  c->d = static_cast<void*>(b + y.d);
   c->macros = reinterpret_cast<double*>(b + y.macros);
   c->cond = reinterpret_cast<int*>(b + y.cond);
   c->aux = reinterpret_cast<double*>(b + y.aux);
@@ -492,8 +484,9 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
   if (e != cudaSuccess) st = set_cuda_error(e);
   if (!st) st = prepare_stencil_kernels();
   if (!st) st = prepare_fft_kernels();
-  if (!st) st = prepare_slab_kernels();
-  c->fused = slab_fits(c) && !std::getenv("PGJ_UNFUSED") ? 1 : 0;
+  if (!st && c->planes) st = planes_prepare(c->planes);
+  c->four = c->planes && !std::getenv("PGJ_UNFUSED") ? 1 : 0;
+  c->fused = c->four && fused_selectable(n, precision) ? 1 : 0;
   if (!st) st = init_fft_tables(c, s);
   if (!st) st = build_symbol(n, lam, mu, c->symbol, c->symbol32, s);
   if (!st) {
@@ -694,17 +687,17 @@ int pgj_solve_wait(pgj_ctx* c, pgj_load_info* info, void* stream) {
     all = all && ok;
   }
   const long long attempts = cnt[4] + 1;
-  // loop body: operator, update, 5 Green passes, p update (fused: operator, fxy, fz, ifxy), plus the
-  // IF-condition kernel of the reliable-update form; the first direction is 6 kernels (fused FP32:
-  // 7, with the FP32 scale copy) after the mask / recurrence-start kernel
-  const long long body = (c->fused ? 4 : 8) + (c->prec == PGJ_FP32 ? 1 : 0);
+  // loop body: operator, update, 5 Green passes, p update (fused: operator and three plane kernels), plus the
+  // IF-condition kernel of the step-by-step reliable-update form; the first direction is 6 kernels after the mask /
+  // recurrence-start kernel, and the plane kernels' FP64 form ends with x += d
+  const long long body = c->four ? 4 : 8 + (c->prec == PGJ_FP32 ? 1 : 0);
   const long long first = first_direction_launches(c);
   if (uses_resident(c))  // scale copy, the resident recurrence, certify, decide
     c->last_launches = 2 + 3 + attempts * (2 + 3 + 1);
   else if (c->prec == PGJ_FP32)  // rel start, first direction, fold, certify, decide; 3 per replacement
     c->last_launches = 2 + 3 + attempts * (1 + first + 1 + 3 + 1) + body * cnt[5] + 3LL * cnt[3];
   else  // init mask, first direction, certify, decide
-    c->last_launches = 2 + 3 + attempts * (1 + first + 3 + 1) + body * cnt[5];
+    c->last_launches = 2 + 3 + attempts * (1 + first + (c->four ? 1 : 0) + 3 + 1) + body * cnt[5];
   c->last_refinements = c->prec == PGJ_FP32 ? 1 + cnt[3] : 1;
   if (cnt[2]) return PGJ_ERR_TIMEOUT;
   if (cnt[1]) return PGJ_ERR_ITERATION_CAP;
@@ -766,7 +759,7 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
       ++sweeps;
       if ((e = read_state(true)) != cudaSuccess) return set_cuda_error(e);
       // sweep: inner start + first direction, loop bodies, x += d, 3 certification kernels
-      launches += 1 + first_direction_launches(c) + (c->fused ? 4LL : 8LL) * body[0] + 1 + 3;
+      launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * body[0] + 1 + 3;
       if (body[1]) { capped_by_bound = true; break; }
     }
   } else {
@@ -774,9 +767,9 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
       if ((e = cudaGraphLaunch(c->graphs->attempt, s)) != cudaSuccess) return set_cuda_error(e);
       if ((e = read_state(true)) != cudaSuccess) return set_cuda_error(e);
       if (c->prec == PGJ_FP32)  // rel start + first direction, bodies, 3 per replacement, fold + certify
-        launches += 1 + first_direction_launches(c) + (c->fused ? 5LL : 9LL) * body[0] + 3LL * body[3] + 1 + 3;
+        launches += 1 + first_direction_launches(c) + (c->four ? 5LL : 9LL) * body[0] + 3LL * body[3] + 1 + 3;
       else  // attempt: init mask + first direction, loop bodies, 3 certification kernels
-        launches += 1 + first_direction_launches(c) + (c->fused ? 4LL : 8LL) * body[0] + 3;
+        launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * body[0] + 3;
       if (body[1]) { capped_by_bound = true; break; }
       bool all, anybad, capped;
       evaluate(all, anybad, capped);
@@ -830,8 +823,8 @@ int pgj_tile_config(pgj_ctx* c, int* out) {
 
 int pgj_set_fused_iteration(pgj_ctx* c, int on) {
   if (!c || (on != 0 && on != 1)) return PGJ_ERR_ARGUMENT;
-  if (on && !slab_fits(c)) return PGJ_ERR_UNSUPPORTED;
-  c->fused = on;
+  if (on && !fused_selectable(c->n, c->prec)) return PGJ_ERR_UNSUPPORTED;
+  c->fused = c->four = on;
   c->graphs->loads = 0;  // rebuild the solve graphs with the other kernel set
   c->graphs->attempt_loads = 0;
   return PGJ_OK;
@@ -872,16 +865,15 @@ int pgj_profile_iteration(pgj_ctx* c, int loads, const double* macros, int reps,
     return st;
   }
   if (!st) st = capture_first_direction(c, loads, s);
-  const bool fused = c->fused != 0;
-  void* u = prec == PGJ_FP32 ? c->d : static_cast<void*>(c->x);
+  const bool fused = c->four != 0;
   cudaEvent_t ev[2 * PGJ_PROFILE_KERNELS];
   for (int k = 0; k < 2 * PGJ_PROFILE_KERNELS; ++k) cudaEventCreate(&ev[k]);
   double acc[PGJ_PROFILE_KERNELS] = {0};
   auto launch_k = [&](int k) -> int {
     if (k == 0) return launch_recurrence_operator(c, loads, prec, s);
-    if (fused && k == 1) return launch_fxy(c, loads, prec, kSlabUpdateL, u, s);
-    if (fused && k == 2) return launch_fz_fused(c, loads, prec, false, s);
-    if (fused && k == 3) return launch_ifxy(c, loads, prec, false, s, 0, false);
+    if (fused && k == 1) return launch_planes_fwd(c, loads, kPlanesUpdate, s);
+    if (fused && k == 2) return launch_planes_z(c, loads, false, s);
+    if (fused && k == 3) return launch_planes_inv(c, loads, false, s, 0, false);
     if (fused) return PGJ_OK;
     if (k == 1) return prec == PGJ_FP32 ? launch_update_ur(c, loads, prec, nullptr, c->d, s)
                                         : launch_update_ur(c, loads, prec, c->x, nullptr, s);
@@ -901,7 +893,7 @@ int pgj_profile_iteration(pgj_ctx* c, int loads, const double* macros, int reps,
   for (int k = 0; k < PGJ_PROFILE_KERNELS && !st; ++k) {
     float t = 0.f;
     cudaEventElapsedTime(&t, ev[2 * k], ev[2 * k + 1]);
-    acc[k] = t;
+    acc[k] = fused && k >= 4 ? 0.0 : t;
   }
   c->scal = c->scal_out;
   for (int k = 0; k < 2 * PGJ_PROFILE_KERNELS; ++k) cudaEventDestroy(ev[k]);
@@ -909,14 +901,13 @@ int pgj_profile_iteration(pgj_ctx* c, int loads, const double* macros, int reps,
   const double sz = prec == PGJ_FP32 ? 4.0 : 8.0;     // bytes per real of the inner precision
   const double V = double(N3) * sz * loads;           // one DOF vector over all loads
   const double S = double(Nh) * 3 * 2 * sz * loads;  // one complex half spectrum over all loads
-  // scale field: FP64, or the FP32 planar copy the fused FP32 slab kernels read
+  // scale field: FP64, or the copy the plane kernels read
   const double sc = double(N3) * ((fused && prec == PGJ_FP32) ? 4.0 : 8.0);
-  const double ub = prec == PGJ_FP32 ? V : 2 * V;   // iterate: FP64 x or the inner-precision correction
   const double fused_algo[PGJ_PROFILE_KERNELS] = {
       2 * V + 8.0 * N,                            // operator: read p (+a), write q
-      4 * V + ub + sc + S,                        // fxy: read p q r (+u +s), write r (+u), write spectrum
-      2 * S + 6.0 * Nh * sz + S / loads,          // fz: spectrum in/out, symbol, DFT(s)
-      S + sc + 2 * V, 0, 0, 0, 0};                // ifxy: read spectrum (+s) and p, write p
+      3 * V + sc + S,                             // forward: read q r (+s), write r, write spectrum
+      2 * S + 6.0 * Nh * sz + S / loads,          // z: spectrum in/out, symbol, DFT(s)
+      S + sc + 4 * V, 0, 0, 0, 0};                // inverse: read spectrum (+s), p and d, write p and d
   const double algo[PGJ_PROFILE_KERNELS] = {
       2 * V + 8.0 * N,                  // operator: read p (+a), write q
       6 * V,                            // update_ur: read u p r q, write u r

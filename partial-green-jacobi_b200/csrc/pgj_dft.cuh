@@ -140,6 +140,34 @@ template <typename T, bool INV> struct Dft<T, 9, INV> {
   }
 };
 
+template <typename T, bool INV> struct Dft<T, 16, INV> {
+  using C = cplx<T>;
+  static __device__ __forceinline__ void run(C (&v)[16]) {
+    // W16^k, k = 1, 2, 3, 6, 9 (forward); W16^4 is a quarter turn
+    const T c1 = T(0.92387953251128675613), s1 = T(0.38268343236508977173), r2 = T(0.70710678118654752440);
+    const T sg = INV ? T(1) : T(-1);
+    const C w1 = cmk<C>(c1, sg * s1), w2 = cmk<C>(r2, sg * r2), w3 = cmk<C>(s1, sg * c1);
+    const C w6 = cmk<C>(-r2, sg * r2), w9 = cmk<C>(-c1, -sg * s1);
+    C g[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[j][i] = v[4 * i + j];
+      Dft<T, 4, INV>::run(g[j]);
+    }
+    g[1][1] = cmul(g[1][1], w1); g[1][2] = cmul(g[1][2], w2); g[1][3] = cmul(g[1][3], w3);
+    g[2][1] = cmul(g[2][1], w2); g[2][2] = rot90<C, INV>(g[2][2]); g[2][3] = cmul(g[2][3], w6);
+    g[3][1] = cmul(g[3][1], w3); g[3][2] = cmul(g[3][2], w6); g[3][3] = cmul(g[3][3], w9);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      C h[4] = {g[0][k], g[1][k], g[2][k], g[3][k]};
+      Dft<T, 4, INV>::run(h);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) v[k + 4 * m] = h[m];
+    }
+  }
+};
+
 // Factors of a line: RA points per pass-A butterfly, RB per pass-B one (the larger first: the passes
 // that also touch global memory are the A passes, and a wider butterfly keeps more loads in flight).
 template <int N> struct Line;
@@ -147,6 +175,8 @@ template <int N> struct Line;
   template <> struct Line<N_> {                                    \
     static constexpr int RA = A_, RB = B_;                         \
   };
+PGJ_LINE(4, 2, 2)
+PGJ_LINE(6, 3, 2)
 PGJ_LINE(8, 4, 2)
 PGJ_LINE(10, 5, 2)
 PGJ_LINE(12, 4, 3)
@@ -163,6 +193,14 @@ PGJ_LINE(50, 10, 5)
 PGJ_LINE(54, 9, 6)
 PGJ_LINE(60, 10, 6)
 PGJ_LINE(64, 8, 8)
+PGJ_LINE(72, 9, 8)
+PGJ_LINE(80, 10, 8)
+PGJ_LINE(90, 10, 9)
+PGJ_LINE(96, 12, 8)
+PGJ_LINE(100, 10, 10)
+PGJ_LINE(108, 12, 9)
+PGJ_LINE(120, 12, 10)
+PGJ_LINE(128, 16, 8)
 #undef PGJ_LINE
 
 // position of wavenumber k of a transformed line

@@ -119,15 +119,7 @@ struct GreenArgs {
   int use_mean;          // subtract scal.mean_r before scaling (projection P of the input)
   int init;              // FZ finalizer: initialise rz instead of forming beta
   int finalize_fz;       // FZ last block forms rz / beta (recurrence use only)
-  // slab-fused recurrence (the x/y transforms run in the PCG update kernels): the spectrum holds
-  // DFT(s.r); FZ subtracts mean_r . shat (shat = DFT(s)) and forms mean(s.w) by Parseval
-  const void* shat;      // (designs, 3, n, n, nsp) complex T: DFT of each component of the scale field
-  int fused;
-  int forward_only;      // FZ: forward transform along z only (builds shat)
-  int unit_input;        // FX: transform s itself (r ignored; builds shat)
-  const float4* axis;    // per-axis symbol factors (m, v, d), FP32 z pass at n = 64
   int flex;              // flexible beta: beta = (rz_new - r_new . z_prev) / rz
-  double lam, mu;
 };
 
 __device__ __forceinline__ bool load_on(const GreenArgs& A, int load) {
@@ -159,7 +151,7 @@ __global__ void __launch_bounds__(512) k_fx(const GreenArgs A) {
     const size_t g = gbase + i;
     const int c = i % 3;
     const T mc = c == 0 ? m[0] : (c == 1 ? m[1] : m[2]);
-    return A.unit_input ? T(sc[g]) : T(sc[g]) * (r[g] - mc);
+    return T(sc[g]) * (r[g] - mc);
   }, [&](int i, T v) {
     const int rl = fdiv(i, A.geo.div_3n);
     const int rem = i - rl * 3 * n;
@@ -245,22 +237,13 @@ __global__ void __launch_bounds__(512) k_fz(const GreenArgs A) {
   __syncthreads();
   const C* tw = reinterpret_cast<const C*>(A.tw);
   C* res = fft_line<T>(b0, b1, kl < kn ? line * pitch : -1, 1, A.plan, tw, false);
-  if (A.forward_only) {
-    if (kl < kn)
-      for (int z = threadIdx.y; z < n; z += blockDim.y)
-        sp[c * plane + (size_t(z) * n + ky) * nsp + k0 + kl] = res[line * pitch + z];
-    return;
-  }
   // symbol multiply and Parseval partial sums: rows kz over (threadIdx.y, threadIdx.z)
   const T* sym = reinterpret_cast<const T*>(A.sym);
-  const C* sh = reinterpret_cast<const C*>(A.shat) + size_t(load / A.lpd) * 3 * plane;
   const size_t Nh = size_t(n) * n * ns;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  double acc[1] = {0.0};
   if (kl < kn) {
     const int kx = k0 + kl;
     const double wgt = (kx == 0 || kx == n / 2) ? 1.0 : 2.0;
-    T m[3] = {T(0), T(0), T(0)};
-    if (A.fused) { m[0] = T(A.scal[load].mean_r[0]); m[1] = T(A.scal[load].mean_r[1]); m[2] = T(A.scal[load].mean_r[2]); }
     for (int kz = threadIdx.y + blockDim.y * threadIdx.z; kz < n; kz += blockDim.y * blockDim.z) {
       const size_t kk = (size_t(kz) * n + ky) * ns + kx;
       const T c0 = sym[kk], c1 = sym[Nh + kk], c2 = sym[2 * Nh + kk];
@@ -269,27 +252,12 @@ __global__ void __launch_bounds__(512) k_fz(const GreenArgs A) {
       C* py = res + (1 * kc + kl) * pitch + kz;
       C* pz = res + (2 * kc + kl) * pitch + kz;
       C x = *px, y = *py, zv = *pz;
-      C s0, s1, s2;
-      if (A.fused) {
-        // DFT(s.(r - mean r)) = DFT(s.r) - mean r . DFT(s)
-        const size_t ks = (size_t(kz) * n + ky) * nsp + kx;
-        s0 = sh[ks]; s1 = sh[plane + ks]; s2 = sh[2 * plane + ks];
-        x.x -= m[0] * s0.x; x.y -= m[0] * s0.y;
-        y.x -= m[1] * s1.x; y.y -= m[1] * s1.y;
-        zv.x -= m[2] * s2.x; zv.y -= m[2] * s2.y;
-      }
       C wx, wy, wz;
       wx.x = c0 * x.x + c3 * y.x + c4 * zv.x; wx.y = c0 * x.y + c3 * y.y + c4 * zv.y;
       wy.x = c3 * x.x + c1 * y.x + c5 * zv.x; wy.y = c3 * x.y + c1 * y.y + c5 * zv.y;
       wz.x = c4 * x.x + c5 * y.x + c2 * zv.x; wz.y = c4 * x.y + c5 * y.y + c2 * zv.y;
       acc[0] += wgt * (double(x.x) * wx.x + double(x.y) * wx.y + double(y.x) * wy.x + double(y.y) * wy.y +
                        double(zv.x) * wz.x + double(zv.y) * wz.y);
-      if (A.fused) {
-        // sum_x s w = sum_k W conj(DFT(s)) (1/N is folded into the symbol)
-        acc[1] += wgt * (double(wx.x) * s0.x + double(wx.y) * s0.y);
-        acc[2] += wgt * (double(wy.x) * s1.x + double(wy.y) * s1.y);
-        acc[3] += wgt * (double(wz.x) * s2.x + double(wz.y) * s2.y);
-      }
       *px = wx; *py = wy; *pz = wz;
     }
   }
@@ -302,22 +270,12 @@ __global__ void __launch_bounds__(512) k_fz(const GreenArgs A) {
   if (!A.finalize_fz) return;
   const int nblk = gridDim.x * gridDim.y, blk = blockIdx.x + gridDim.x * blockIdx.y;
   double* part = A.partials + size_t(load) * kPartialQ * kMaxPartials;
-  if (A.fused) {
-    block_sum<4>(acc, red);
-    if (tid == 0)
-      for (int k = 0; k < 4; ++k) part[k * kMaxPartials + blk] = acc[k];
-  } else {
-    double a1[1] = {acc[0]};
-    block_sum<1>(a1, red);
-    if (tid == 0) part[blk] = a1[0];
-  }
+  block_sum<1>(acc, red);
+  if (tid == 0) part[blk] = acc[0];
   LoadScalars& S = A.scal[load];
   if (!last_block(&S.ticket[kTicketFZ], nblk)) return;
   if (tid < 32) {
     const double rzn = warp_sum_partials(part, nblk);
-    double mz[3] = {0.0, 0.0, 0.0};
-    if (A.fused)
-      for (int k = 0; k < 3; ++k) mz[k] = warp_sum_partials(part + (k + 1) * kMaxPartials, nblk);
     if (tid == 0) {
       if (A.init) {
         S.beta = 0.0;
@@ -326,187 +284,6 @@ __global__ void __launch_bounds__(512) k_fz(const GreenArgs A) {
         S.beta = (A.flex ? rzn - S.rz_cross : rzn) / (rz != 0.0 ? rz : 1.0);
       }
       S.rz = rzn;
-      if (A.fused)
-        for (int k = 0; k < 3; ++k) S.mean_z[k] = mz[k] / double(size_t(n) * n * n);
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------- FZ, n = 64
-// z pass of the fused recurrence at n = 64 with the line transforms in registers: a 64-point line
-// is an 8 x 8 four-step transform. Lane a of the 8 lanes of a line holds points z = a + 8b; it does
-// the 8-point DFT over b, multiplies by w64^(a k2), and a transpose through this warp's shared
-// memory hands lane t the values with k2 = t for the 8-point DFT over a; lane t then owns
-// kz = t + 8 k1. The inverse runs the same steps backwards. A warp owns four kx columns at one ky
-// (all three components); warps never wait on each other, so the only block barrier is the final
-// reduction. Same results as k_fz in fused mode (rz, beta and mean(s.w) by Parseval).
-constexpr int kFz64Line = 72;                 // complex slots per line (8 rows of 9; conflict-free, as kLine64)
-
-// The FI symbol at (kx, ky, kz) from the per-axis factors (m, v, d) of each wavenumber, the same
-// algebra as k_symbol: t = h^3 prod m, trace = t sum (d + v^2), inv_i = 1/(mu trace + (lam+mu) t d_i),
-// beta = (lam+mu) t / (1 + sum (lam+mu) t v_i^2 inv_i), cf = (diag(inv) - beta w w^T) / N, w_i = inv_i v_i.
-// In FP32 it replaces six scattered loads per wavevector by a few arithmetic instructions.
-__device__ __forceinline__ void fi_symbol_f32(const float4& ax, const float4& ay, const float4& az, bool origin,
-                                              float lam, float mu, float h3, float invN, float (&cf)[6]) {
-  float t = h3 * ax.x;
-  t *= ay.x;
-  t *= az.x;
-  const float trace = ((ax.z + ax.y * ax.y) + (ay.z + ay.y * ay.y) + (az.z + az.y * az.y)) * t;
-  const float lm = lam + mu, b = lm * t;
-  const float inv0 = origin ? 0.f : __frcp_rn(mu * trace + b * ax.z);
-  const float inv1 = origin ? 0.f : __frcp_rn(mu * trace + b * ay.z);
-  const float inv2 = origin ? 0.f : __frcp_rn(mu * trace + b * az.z);
-  const float den = 1.f + b * ax.y * ax.y * inv0 + b * ay.y * ay.y * inv1 + b * az.y * az.y * inv2;
-  const float beta = origin ? 0.f : __fdiv_rn(b, den);
-  const float w0 = inv0 * ax.y, w1 = inv1 * ay.y, w2 = inv2 * az.y;
-  cf[0] = (inv0 - beta * w0 * w0) * invN;
-  cf[1] = (inv1 - beta * w1 * w1) * invN;
-  cf[2] = (inv2 - beta * w2 * w2) * invN;
-  cf[3] = -beta * w0 * w1 * invN;
-  cf[4] = -beta * w0 * w2 * invN;
-  cf[5] = -beta * w1 * w2 * invN;
-}
-constexpr int kFz64Comp = 4 * kFz64Line;      // one component of the warp's four lines
-
-template <typename T, int WPB, int MINB>
-__global__ void __launch_bounds__(WPB * 32, MINB) k_fz64(const GreenArgs A) {
-  using C = cplx<T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int N = 64;
-  const int load = blockIdx.y;
-  if (!load_on(A, load)) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int l = lane >> 3, t = lane & 7;
-  const int ns = A.ns, nsp = A.nsp;
-  const int groups = (ns + 3) >> 2;
-  const int w = blockIdx.x * WPB + warp;
-  const int ky = w / groups, kx = (w - ky * groups) * 4 + l;
-  const bool valid = ky < N && kx < ns;
-  C* buf = reinterpret_cast<C*>(smem_raw) + (warp * 3 * 4 + l) * kFz64Line;  // + c * kFz64Comp
-  double* red = reinterpret_cast<double*>(reinterpret_cast<C*>(smem_raw) + WPB * 3 * kFz64Comp);
-  const size_t plane = size_t(N) * N * nsp;
-  C* sp = reinterpret_cast<C*>(A.spec) + size_t(load) * 3 * plane;
-  const C* tw = reinterpret_cast<const C*>(A.tw);
-  const C zero = cmk<C>(0.0, 0.0);
-  const size_t col = size_t(ky) * nsp + kx;  // offset of (z = 0, ky, kx) in one component
-  // forward: DFT over b, twiddle, column write (row k2, column t)
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    C v[8];
-#pragma unroll
-    for (int b = 0; b < 8; ++b) v[b] = valid ? sp[c * plane + size_t(t + 8 * b) * N * nsp + col] : zero;
-    Radix<T, 8>::run(v, false);
-#pragma unroll
-    for (int k2 = 1; k2 < 8; ++k2) v[k2] = cmul(v[k2], __ldg(&tw[t * k2]));
-#pragma unroll
-    for (int k2 = 0; k2 < 8; ++k2) buf[c * kFz64Comp + k2 * 9 + t] = v[k2];
-  }
-  __syncwarp();
-  // DFT over a of row t; X[kz = t + 8 k1] goes to (row k1, column t)
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    C v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = buf[c * kFz64Comp + t * 9 + j];
-    Radix<T, 8>::run(v, false);
-    __syncwarp();  // every lane has read its row before the column writes
-#pragma unroll
-    for (int k1 = 0; k1 < 8; ++k1) buf[c * kFz64Comp + k1 * 9 + t] = v[k1];
-  }
-  // symbol multiply and the Parseval sums on the lane's own column
-  const T* sym = reinterpret_cast<const T*>(A.sym);
-  const C* sh = reinterpret_cast<const C*>(A.shat) + size_t(load / A.lpd) * 3 * plane;
-  const size_t Nh = size_t(N) * N * ns;
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  if (valid) {
-    const double wgt = (kx == 0 || kx == N / 2) ? 1.0 : 2.0;
-    const T m0 = T(A.scal[load].mean_r[0]), m1 = T(A.scal[load].mean_r[1]), m2 = T(A.scal[load].mean_r[2]);
-    float4 axx = make_float4(0.f, 0.f, 0.f, 0.f), axy = axx;
-    const float h3 = 1.f / float(N * N * N), invN = h3;
-    if constexpr (sizeof(T) == 4) { axx = A.axis[kx]; axy = A.axis[ky]; }
-#pragma unroll 2
-    for (int k1 = 0; k1 < 8; ++k1) {
-      const int kz = t + 8 * k1;
-      T c0, c1, c2, c3, c4, c5;
-      if constexpr (sizeof(T) == 4) {
-        float cf[6];
-        fi_symbol_f32(axx, axy, A.axis[kz], kx == 0 && ky == 0 && kz == 0, float(A.lam), float(A.mu), h3, invN, cf);
-        c0 = cf[0]; c1 = cf[1]; c2 = cf[2]; c3 = cf[3]; c4 = cf[4]; c5 = cf[5];
-      } else {
-        const size_t kk = (size_t(kz) * N + ky) * ns + kx;
-        c0 = sym[kk]; c1 = sym[Nh + kk]; c2 = sym[2 * Nh + kk];
-        c3 = sym[3 * Nh + kk]; c4 = sym[4 * Nh + kk]; c5 = sym[5 * Nh + kk];
-      }
-      const size_t ks = size_t(kz) * N * nsp + col;
-      const C s0 = sh[ks], s1 = sh[plane + ks], s2 = sh[2 * plane + ks];
-      C* px = buf + k1 * 9 + t;
-      C x = px[0], y = px[kFz64Comp], zv = px[2 * kFz64Comp];
-      x.x -= m0 * s0.x; x.y -= m0 * s0.y;
-      y.x -= m1 * s1.x; y.y -= m1 * s1.y;
-      zv.x -= m2 * s2.x; zv.y -= m2 * s2.y;
-      C wx, wy, wz;
-      wx.x = c0 * x.x + c3 * y.x + c4 * zv.x; wx.y = c0 * x.y + c3 * y.y + c4 * zv.y;
-      wy.x = c3 * x.x + c1 * y.x + c5 * zv.x; wy.y = c3 * x.y + c1 * y.y + c5 * zv.y;
-      wz.x = c4 * x.x + c5 * y.x + c2 * zv.x; wz.y = c4 * x.y + c5 * y.y + c2 * zv.y;
-      acc[0] += wgt * (double(x.x) * wx.x + double(x.y) * wx.y + double(y.x) * wy.x + double(y.y) * wy.y +
-                       double(zv.x) * wz.x + double(zv.y) * wz.y);
-      acc[1] += wgt * (double(wx.x) * s0.x + double(wx.y) * s0.y);
-      acc[2] += wgt * (double(wy.x) * s1.x + double(wy.y) * s1.y);
-      acc[3] += wgt * (double(wz.x) * s2.x + double(wz.y) * s2.y);
-      px[0] = wx; px[kFz64Comp] = wy; px[2 * kFz64Comp] = wz;
-    }
-  }
-  // inverse: DFT over k1 of the own column, twiddle, column write (row a, column t); then the
-  // DFT over k2 of row t gives z = t + 8 b
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    C v[8];
-#pragma unroll
-    for (int k1 = 0; k1 < 8; ++k1) v[k1] = buf[c * kFz64Comp + k1 * 9 + t];
-    Radix<T, 8>::run(v, true);
-#pragma unroll
-    for (int a = 1; a < 8; ++a) {
-      C wt = __ldg(&tw[t * a]);
-      wt.y = -wt.y;
-      v[a] = cmul(v[a], wt);
-    }
-#pragma unroll
-    for (int a = 0; a < 8; ++a) buf[c * kFz64Comp + a * 9 + t] = v[a];
-  }
-  __syncwarp();
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    C v[8];
-#pragma unroll
-    for (int k2 = 0; k2 < 8; ++k2) v[k2] = buf[c * kFz64Comp + t * 9 + k2];
-    Radix<T, 8>::run(v, true);
-    if (valid) {
-#pragma unroll
-      for (int b = 0; b < 8; ++b) sp[c * plane + size_t(t + 8 * b) * N * nsp + col] = v[b];
-    }
-  }
-  // Parseval partials -> last block: rz, beta, mean(s.w) (as k_fz)
-  const int tid = threadIdx.x;
-  block_sum<4>(acc, red);
-  const int nblk = gridDim.x, blk = blockIdx.x;
-  double* part = A.partials + size_t(load) * kPartialQ * kMaxPartials;
-  if (tid == 0)
-    for (int k = 0; k < 4; ++k) part[k * kMaxPartials + blk] = acc[k];
-  LoadScalars& S = A.scal[load];
-  if (!last_block(&S.ticket[kTicketFZ], nblk)) return;
-  if (tid < 32) {
-    const double rzn = warp_sum_partials(part, nblk);
-    double mz[3];
-    for (int k = 0; k < 3; ++k) mz[k] = warp_sum_partials(part + (k + 1) * kMaxPartials, nblk);
-    if (tid == 0) {
-      if (A.init) {
-        S.beta = 0.0;
-      } else {
-        const double rz = S.rz;
-        S.beta = (A.flex ? rzn - S.rz_cross : rzn) / (rz != 0.0 ? rz : 1.0);
-      }
-      S.rz = rzn;
-      for (int k = 0; k < 3; ++k) S.mean_z[k] = mz[k] / double(size_t(N) * N * N);
     }
   }
 }
@@ -601,25 +378,6 @@ static size_t smem_x(const pgj_ctx* c, size_t cb) {
 static size_t smem_y(const pgj_ctx* c, size_t cb) { return 2 * size_t(c->fg.kcy) * (c->n + 1) * cb; }
 static size_t smem_z(const pgj_ctx* c, size_t cb) { return 2 * 3 * size_t(c->fg.kcz) * (c->n + 1) * cb + 32 * 4 * 8 + 64; }
 
-template <typename T> constexpr int fz64_warps() { return sizeof(T) == 4 ? 8 : 4; }  // warps per block
-template <typename T>
-static size_t fz64_smem() { return size_t(fz64_warps<T>()) * 3 * kFz64Comp * 2 * sizeof(T) + 32 * 4 * 8 + 64; }
-
-template <typename T>
-static int run_fz64(pgj_ctx* c, int loads, const GreenArgs& A, cudaStream_t s) {
-  constexpr int WPB = fz64_warps<T>();
-  const int warps = ((c->ns + 3) / 4) * c->n;  // per load
-  const dim3 grid((warps + WPB - 1) / WPB, loads);
-  // blocks per SM the register budget is sized for: default three; PGJ_FZ64_MINB = 1 (unbounded), 4, 6
-  const char* e = std::getenv("PGJ_FZ64_MINB");
-  const int minb = e ? std::atoi(e) : 3;
-  if (minb == 1) k_fz64<T, WPB, 1><<<grid, WPB * 32, fz64_smem<T>(), s>>>(A);
-  else if (minb == 4) k_fz64<T, WPB, 4><<<grid, WPB * 32, fz64_smem<T>(), s>>>(A);
-  else if (minb == 6) k_fz64<T, WPB, 6><<<grid, WPB * 32, fz64_smem<T>(), s>>>(A);
-  else k_fz64<T, WPB, 3><<<grid, WPB * 32, fz64_smem<T>(), s>>>(A);
-  return check_launch();
-}
-
 template <typename T>
 static int set_smem_limits() {
   const int lim = 220 * 1024;  // below the 227 KB opt-in less the static shared memory
@@ -628,10 +386,6 @@ static int set_smem_limits() {
   cudaFuncSetAttribute(k_fy<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_fz<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_ifx<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fz64<T, fz64_warps<T>(), 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fz64<T, fz64_warps<T>(), 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fz64<T, fz64_warps<T>(), 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_fz64<T, fz64_warps<T>(), 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   return check_launch();
 }
 
@@ -664,10 +418,6 @@ static int run_green(pgj_ctx* c, int loads, GreenArgs& A, cudaStream_t s) {
   return PGJ_OK;
 }
 
-static float4* axis_table(pgj_ctx* c) {
-  return reinterpret_cast<float4*>(static_cast<char*>(c->tw) + size_t(c->n) * (sizeof(double2) + sizeof(float2)));
-}
-
 static GreenArgs green_args(pgj_ctx* c, int prec, const void* r) {
   GreenArgs A;
   std::memset(&A, 0, sizeof(A));
@@ -677,8 +427,6 @@ static GreenArgs green_args(pgj_ctx* c, int prec, const void* r) {
   A.sym = prec == PGJ_FP32 ? static_cast<const void*>(c->symbol32) : static_cast<const void*>(c->symbol);
   A.tw = prec == PGJ_FP32 ? static_cast<const void*>(static_cast<double2*>(c->tw) + c->n) : c->tw;
   A.sw = c->sw; A.scal = c->scal; A.partials = c->partials;
-  A.axis = axis_table(c);
-  A.lam = c->lam; A.mu = c->mu;
   A.flex = prec == PGJ_FP32 ? c->flex : 0;  // beta of the FP32 recurrence: flexible form when set
   return A;
 }
@@ -699,37 +447,6 @@ int launch_green(pgj_ctx* c, int loads, int prec, const void* r, bool init, cuda
   A.init = init ? 1 : 0;
   A.finalize_fz = 1;
   return prec == PGJ_FP32 ? run_green<float>(c, loads, A, s) : run_green<double>(c, loads, A, s);
-}
-
-// z pass of the slab-fused iteration (DFT(s.r) in the spectrum; mean r subtracted through shat).
-int launch_fz_fused(pgj_ctx* c, int loads, int prec, bool init, cudaStream_t s) {
-  GreenArgs A = green_args(c, prec, c->r);
-  A.skip_inactive = 1;
-  A.init = init ? 1 : 0;
-  A.finalize_fz = 1;
-  A.fused = 1;
-  A.shat = c->shat;
-  const char* e = std::getenv("PGJ_FZ64");
-  if (c->n == 64 && !(e && e[0] == '0'))  // line transforms in registers (PGJ_FZ64=0: generic pass)
-    return prec == PGJ_FP32 ? run_fz64<float>(c, loads, A, s) : run_fz64<double>(c, loads, A, s);
-  return prec == PGJ_FP32 ? run_green_pass<float>(c, loads, A, s, 2) : run_green_pass<double>(c, loads, A, s, 2);
-}
-
-// shat = DFT(s) per component (in the context precision), through the x, y and forward z passes on
-// the spectrum of load 0; called whenever the scale field changes.
-int build_shat(pgj_ctx* c, cudaStream_t s) {
-  GreenArgs A = green_args(c, c->prec, c->r);
-  A.skip_inactive = 0;
-  A.use_mean = 0;
-  A.unit_input = 1;
-  A.forward_only = 1;
-  for (int pass = 0; pass < 3; ++pass) {
-    const int st = c->prec == PGJ_FP32 ? run_green_pass<float>(c, 1, A, s, pass) : run_green_pass<double>(c, 1, A, s, pass);
-    if (st) return st;
-  }
-  const size_t bytes = 2 * size_t(c->prec == PGJ_FP32 ? 4 : 8) * 3 * size_t(c->n) * c->n * (c->ns + (c->ns & 1));
-  const cudaError_t e = cudaMemcpyAsync(c->shat, c->spec, bytes, cudaMemcpyDeviceToDevice, s);
-  return e == cudaSuccess ? PGJ_OK : set_cuda_error(e);
 }
 
 // z = P(s . w) = s.w - mean(s.w), from the sw buffer and the IFX finalizer's means.
@@ -844,20 +561,9 @@ int init_fft_tables(pgj_ctx* c, cudaStream_t s) {
     t64[k] = make_double2(cr, ci);
     t32[k] = make_float2((float)cr, (float)ci);
   }
-  // per-axis factors of the FI symbol (the same expressions as k_symbol): m = cos^2 + sin^2/3,
-  // v = 2 sin cos / (h m), d = 4 sin^4 / (3 h^2 m^2) at the half angle pi k / n
-  std::vector<float4> ax(n);
-  const double h = 1.0 / n;
-  for (int k = 0; k < n; ++k) {
-    const double a = 3.14159265358979323846 * k / n, sn = std::sin(a), cs = std::cos(a);
-    const double m = cs * cs + sn * sn / 3;
-    ax[k] = make_float4(float(m), float(2 * sn * cs / (h * m)), float(4 * (sn * sn) * (sn * sn) / (3 * h * h * m * m)), 0.f);
-  }
   cudaError_t e = cudaMemcpyAsync(c->tw, t64.data(), n * sizeof(double2), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(static_cast<double2*>(c->tw) + n, t32.data(), n * sizeof(float2), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(axis_table(c), ax.data(), n * sizeof(float4), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e == cudaSuccess ? PGJ_OK : set_cuda_error(e);
 }

@@ -141,71 +141,4 @@ __device__ cplx<T>* fft_line(cplx<T>* b0, cplx<T>* b1, int off, int es, const FF
   return src;
 }
 
-
-// Stage over `nl` lines at offsets l * lp (elements at stride es), work items w = tid, tid+nthr, ...
-// LFAST: w -> (l = w % nl, j = w / nl); otherwise (l = w / nb, j = w % nb).
-template <typename T, int R, bool LFAST>
-__device__ __forceinline__ void stage_lines(const cplx<T>* __restrict__ src, cplx<T>* __restrict__ dst, int nl, int lp,
-                                            int es, int n, int Ns, const FastDiv& nsd, const FastDiv& div,
-                                            const cplx<T>* __restrict__ tw, bool inv, int tid, int nthr) {
-  using C = cplx<T>;
-  const int nb = n / R;
-  const int step = n / (Ns * R);
-  const int total = nl * nb;
-  for (int w = tid; w < total; w += nthr) {
-    int l, j;
-    if (LFAST) { j = fdiv(w, div); l = w - j * nl; }
-    else { l = fdiv(w, div); j = w - l * nb; }
-    const int jq = fdiv(j, nsd);
-    const int jm = j - jq * Ns;
-    const C* s = src + l * lp;
-    C* d = dst + l * lp;
-    C v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = s[(j + r * nb) * es];
-    if (jm) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) {
-        C w2 = __ldg(&tw[r * jm * step]);
-        if (inv) w2.y = -w2.y;
-        v[r] = cmul(v[r], w2);
-      }
-    }
-    Radix<T, R>::run(v, inv);
-    const int base = jq * Ns * R + jm;
-#pragma unroll
-    for (int r = 0; r < R; ++r) d[(base + r * Ns) * es] = v[r];
-  }
-}
-
-// All stages over `nl` lines, ping-pong between b0 and b1 with one block barrier per stage; returns
-// the buffer holding the result. `ldiv` divides by nl (LFAST only).
-// Always inlined into the slab kernels, its only callers: as a called function it kept their
-// registers and the plan in local memory across the call (a 440-byte stack frame) and made their
-// speed depend on how many kernels called it (slab update n = 32: 16.5 vs 24.5 us). The per-line
-// fft_line of the unfused passes stays a compiler choice (forced inline it made the z pass slower).
-template <typename T, bool LFAST>
-__device__ __forceinline__ cplx<T>* fft_lines(cplx<T>* b0, cplx<T>* b1, int nl, int lp, int es, const FFTPlan& pl,
-                              const FastDiv& ldiv, const cplx<T>* tw, bool inv, int tid, int nthr) {
-  cplx<T>* src = b0;
-  cplx<T>* dst = b1;
-  int Ns = 1;
-  for (int st = 0; st < pl.nst; ++st) {
-    const int R = pl.radix[st];
-    const FastDiv& nsd = pl.ns_div[st];
-    const FastDiv& div = LFAST ? ldiv : pl.nb_div[st];
-    switch (R) {
-      case 8: stage_lines<T, 8, LFAST>(src, dst, nl, lp, es, pl.n, Ns, nsd, div, tw, inv, tid, nthr); break;
-      case 4: stage_lines<T, 4, LFAST>(src, dst, nl, lp, es, pl.n, Ns, nsd, div, tw, inv, tid, nthr); break;
-      case 2: stage_lines<T, 2, LFAST>(src, dst, nl, lp, es, pl.n, Ns, nsd, div, tw, inv, tid, nthr); break;
-      case 3: stage_lines<T, 3, LFAST>(src, dst, nl, lp, es, pl.n, Ns, nsd, div, tw, inv, tid, nthr); break;
-      default: stage_lines<T, 5, LFAST>(src, dst, nl, lp, es, pl.n, Ns, nsd, div, tw, inv, tid, nthr); break;
-    }
-    __syncthreads();
-    cplx<T>* t = src; src = dst; dst = t;
-    Ns *= R;
-  }
-  return src;
-}
-
 }  // namespace pgj

@@ -78,6 +78,7 @@ struct Layout {
 
 struct Graphs;
 struct ResidentKernel;
+struct PlaneKernels;
 
 }  // namespace pgj
 
@@ -111,18 +112,20 @@ struct pgj_ctx {
   void* qb;            // FP32 contexts at n = 64: (L, n, n / hg.ty, 3, n) boundary rows of the halo-free operator
   pgj::StencilGeom hg; // halo-free recurrence operator geometry (FP32 slab-fused contexts)
   int hf;              // FP32 slab-fused recurrences use the halo-free operator (PGJ_HF=0: the halo form)
-  void* sw;            // (L, 3N) T  s . w (unprojected preconditioned residual)
-  void* spec;          // (L, 3, n, n, nsp) complex T
+  void* sw;            // (L, 3N) T  s . w (unprojected preconditioned residual); plane kernels in FP64: the residual
+  void* spec;          // (L, 3, n, n, nsp) complex T (plane kernels: rows of ns)
   void* shat;          // (D, 3, n, n, nsp) complex T: DFT of each component of the scale field
-  double* scale_pl;    // FP64 contexts with a cluster-resident PCG: (D, 3, N) copy of scale by component
+  double* scale_pl;    // FP64 contexts: (D, 3, N) copy of scale by component
   char* halo;          // per load, the planes its cluster's blocks hand to each other
   const pgj::ResidentKernel* res;  // cluster-resident PCG of this grid and precision, or null
-  int fused;           // PCG iteration as operator + slab-fused update/transform kernels
+  const pgj::PlaneKernels* planes; // plane transform kernels of this grid and precision, or null
+  int four;            // PCG iteration as operator + plane transform kernels (or the resident kernel)
+  int fused;           // pgj_fused_iteration: the four-kernel set is selected, on a grid where it may be
   double* partials;    // (L, kPartialQ * kMaxPartials)
   pgj::LoadScalars* scal;  // L records used by the kernels being launched (outer or inner)
   pgj::LoadScalars* scal_out;  // certification / FP64 recurrence records
   pgj::LoadScalars* scal_in;   // mixed refinement: inner FP32 recurrence records
-  void* d;             // mixed: (L, 3N) T inner correction
+  void* d;             // (L, 3N) T correction of the current attempt
   double* macros;      // (L, 6) device copy
   int* cond;           // device flags (any active)
   double* r64;         // mixed: fp64 residual (L, 3N)
@@ -148,7 +151,7 @@ struct pgj_ctx {
 
 namespace pgj {
 // operator (pgj_operator.cu)
-// planar_plain: plain mode writing q component-planar, as the recurrence operator of a slab-fused FP32
+// planar_plain: plain mode writing q component-planar, as the recurrence operator of an FP32
 // context does (the tuner)
 int launch_stencil(pgj_ctx* c, int mode, int loads, int prec, const void* in, void* out, const double* f,
                    const int32_t* active_ext, cudaStream_t s, const LoadScalars* rel_flags = nullptr,
@@ -169,28 +172,27 @@ int launch_green(pgj_ctx* c, int loads, int prec, const void* r, bool init, cuda
 // one Green pass: 0 fft_x, 1 fft_y, 2 fft_z+symbol, 3 ifft_y, 4 ifft_x
 int launch_green_pass(pgj_ctx* c, int loads, int prec, const void* r, bool init, int pass, cudaStream_t s);
 int launch_green_standalone(pgj_ctx* c, int loads, const double* r, double* z, cudaStream_t s);
-int launch_fz_fused(pgj_ctx* c, int loads, int prec, bool init, cudaStream_t s);
-int build_shat(pgj_ctx* c, cudaStream_t s);
-// FP32 contexts: scale32 = float(scale), component-planar (pgj_operator.cu)
-int launch_scale32(pgj_ctx* c, cudaStream_t s);
-// slab-fused iteration (pgj_slab.cu)
-enum SlabLaunch { kSlabUpdateL = 0, kSlabInitL = 1, kSlabSyncL = 2 };
-bool slab_fits(const pgj_ctx* c);
-bool slab_fits_shape(int n, int prec);
+// plane transform kernels (pgj_planes.cu)
+enum PlanesMode { kPlanesUpdate = 0, kPlanesInit = 1, kPlanesSync = 2, kPlanesScale = 3 };
+const PlaneKernels* planes_find(int n, int prec);
+int planes_prepare(const PlaneKernels* k);
+// grids on which pgj_set_fused_iteration selects between the two kernel sets: two planes of transform
+// buffers per SM (up to n = 80 in FP64, 108 in FP32). Larger grids whose plane pair fits one block per SM run
+// the plane kernels as well, but report and accept only 0.
+bool fused_selectable(int n, int prec);
+int launch_planes_fwd(pgj_ctx* c, int loads, int mode, cudaStream_t s, cudaGraphConditionalHandle hif = 0);
+int launch_planes_z(pgj_ctx* c, int loads, bool init, cudaStream_t s);
+int launch_planes_inv(pgj_ctx* c, int loads, bool init, cudaStream_t s, cudaGraphConditionalHandle h, bool set_cond);
+int launch_planes_shat(pgj_ctx* c, int loads, cudaStream_t s);
+// copies the scale fields of the loads' designs by component, in the context precision (pgj_resident.cu)
+int launch_scale_planes(pgj_ctx* c, int loads, cudaStream_t s);
 // halo-free FP32 recurrence operator (pgj_operator.cu): geometry, launch, and whether a context's
-// recurrence uses it (FP32, slab-fused, FP32 arithmetic, not switched off)
+// recurrence uses it (FP32, plane kernels, FP32 arithmetic, not switched off)
 StencilGeom hf_geom(int n, int lpd);
 int launch_stencil_hf(pgj_ctx* c, int loads, cudaStream_t s);
-bool slab_register_path(const pgj_ctx* c, int prec);  // the n = 64 register-transform slab kernels
-inline bool uses_hf(const pgj_ctx* c, int prec) {
-  return prec == PGJ_FP32 && c->fused && c->hf && !c->op64 && slab_register_path(c, prec);
-}
+inline bool uses_hf(const pgj_ctx* c, int prec) { return prec == PGJ_FP32 && c->four && c->hf && !c->op64; }
 // the recurrence operator q = K p (and alpha = r.z / p.q) of one PCG iteration
 int launch_recurrence_operator(pgj_ctx* c, int loads, int prec, cudaStream_t s);
-int prepare_slab_kernels();
-int launch_fxy(pgj_ctx* c, int loads, int prec, int mode, void* u, cudaStream_t s);
-int launch_ifxy(pgj_ctx* c, int loads, int prec, bool init, cudaStream_t s, cudaGraphConditionalHandle h,
-                bool set_cond);
 // cluster-resident PCG (pgj_resident.cu): a whole attempt's recurrence in one launch
 const ResidentKernel* resident_prepare(int n, int prec);
 size_t resident_halo_bytes(int n, int prec);
@@ -198,13 +200,14 @@ int launch_resident(pgj_ctx* c, int loads, cudaStream_t s);
 // The resident kernel runs the plain recurrences: the flexible direction update, FP64 arithmetic on FP32
 // vectors and the refinement sweeps keep the separate kernels, as does a context set to step-by-step.
 inline bool uses_resident(const pgj_ctx* c) {
-  return c->res && c->fused && !c->flex && !c->op64 && !(c->prec == PGJ_FP32 && c->mixed_mode == 1);
+  return c->res && c->four && !c->flex && !c->op64 && !(c->prec == PGJ_FP32 && c->mixed_mode == 1);
 }
 // pcg (pgj_pcg.cu)
 int launch_update_ur(pgj_ctx* c, int loads, int prec, double* u64, void* uT, cudaStream_t s);
 int launch_update_p(pgj_ctx* c, int loads, int prec, bool init, cudaStream_t s, cudaGraphConditionalHandle h,
                     bool set_cond);
 int launch_init_mask(pgj_ctx* c, int loads, cudaStream_t s);
+int launch_fold64(pgj_ctx* c, int loads, cudaStream_t s);
 // mixed refinement (pgj_pcg.cu): inner residual r = T(r64), d = 0, inner targets and masks;
 // then x += d for the loads solved in this sweep
 int launch_inner_start(pgj_ctx* c, int loads, double inner_rtol, cudaStream_t s);
@@ -219,14 +222,12 @@ int launch_rel_sync(pgj_ctx* c, int loads, cudaStream_t s);
 int launch_energies(pgj_ctx* c, int loads, const double* u, const double* macros_dev, double* e, cudaStream_t s);
 int launch_effective_tensor(pgj_ctx* c, const double* a, const double* u, double* C, double* e, cudaStream_t s);
 
-// Points the context's per-design views (a, scale, scale32, shat) at design d for the lifetime of
-// the scope, so that the single-design launchers (scale build, FP32 scale copy, DFT(s)) run on it.
+// Points the context's per-design views (a, scale) at design d for the lifetime of the scope, so that the
+// single-design scale build runs on it.
 struct DesignScope {
   pgj_ctx* c;
   double* a;
   double* scale;
-  float* scale32;
-  void* shat;
   DesignScope(pgj_ctx* ctx, int d);
   ~DesignScope();
 };

@@ -38,7 +38,7 @@ __device__ __forceinline__ void cp_wait_one() { asm volatile("cp.async.wait_grou
 // The rows of one plane issued by the lanes of one warp in parallel (lane r: rows r, r+32, ...):
 // lane 0 arms the mbarrier for all rows first. Called by all 32 lanes of the warp. One copy per node
 // row of 3n interleaved values, landing as [row][x][component]. (The component-planar FP32 vectors
-// of slab-fused contexts are the recurrence's r, d and q; the operator's input p stays interleaved:
+// of the plane kernels are the recurrence's r, d and q; the operator's input p stays interleaved:
 // staging a planar p as three component copies per plane measured 59.5 against 46.0 us.)
 template <typename T>
 __device__ __forceinline__ void tma_plane_warp(T* buf, const T* in, int pz, int y0, int rows, int n, uint64_t* bar,
@@ -173,7 +173,7 @@ __device__ __forceinline__ void face_modes(const T* buf, int row, int x, int n, 
 // high-contrast designs whose FP32 node sums cancel).
 //
 // PL: q of this launch is written component-planar, (3, N) per load (the FP32 recurrence vector of a
-// slab-fused mixed context, read per component by the slab kernels); otherwise node-major with the
+// context on the plane kernels, read per component); otherwise node-major with the
 // components interleaved. p is read interleaved either way.
 template <typename T, int MODE, int OCC, typename R = T, bool PL = false>
 __global__ void __launch_bounds__(OCC == 1 ? 512 : 256, OCC) k_stencil(const StencilArgs A) {
@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(OCC == 1 ? 512 : 256, OCC) k_stencil(const Ste
   if (MODE == kResidual && A.scal[load].frozen) act = false;
   T* out = reinterpret_cast<T*>(A.out) + size_t(load) * 3 * N;
   if (!act) {
+    if (MODE == kPCG && blk == 0 && tid == 0) A.scal[load].step = 0;  // its last step has been taken
     if (MODE == kPlain && out_row) {
       for (int z = z0; z < z0 + zc; ++z) {
         const size_t node = (size_t(z) * n + ey) * n + tx;
@@ -562,16 +563,16 @@ __global__ void __launch_bounds__(OCC == 1 ? 512 : 256, OCC) k_stencil(const Ste
 }
 
 // ------------------------------------------------------------------ halo-free recurrence operator
-// The FP32 recurrence operator of slab-fused mixed contexts, without the halo element row of
+// The FP32 recurrence operator of mixed contexts on the plane kernels, without the halo element row of
 // k_stencil: a block owns TY node rows (TY divides n) and exactly the TY element rows whose lower
 // node row is one of them, so no element is computed twice. Thread (x, ty) owns element (x, y0 + ty).
 // A node row y0 + ty, ty >= 1, gets all four corner contributions inside the block (same order as
 // k_stencil) and is stored. The first row y0 of a tile gets its own elements' corners here; those of
 // the element row below the tile are the upper corners of the top element row of the tile below, which
 // that block writes, per z-plane and tile, to the boundary array qb ([load][z][tile][component][x]);
-// the slab update (k_fxy) adds qb to q on the rows y % TY == 0 as it reads q. (Adding the two parts
+// the update (k_planes_fwd) adds qb to q on the rows y % TY == 0 as it reads q. (Adding the two parts
 // atomically onto zeroed rows of q instead measured slower: the atomics cost the operator 4.6 us and
-// re-zeroing the rows cost the slab update 4 us.) p^T q counts each part in the block that computes
+// re-zeroing the rows cost the update 4 us.) p^T q counts each part in the block that computes
 // it, with p of the node it belongs to (the upper face of the top row), so alpha = r.z / p^T q is the
 // quantity of the halo form; only the rounding of the first rows differs.
 // Planes are staged as TY + 1 node rows (y0 .. y0 + TY), q is written component-planar, p is read
@@ -606,7 +607,10 @@ __global__ void __launch_bounds__(256, 2) k_stencil_hf(const StencilArgs A) {
   const int zc = min(A.zc, n - z0);
   const int ey = y0 + ty;  // element row = own node row (< n: TY divides n)
   LoadScalars& S = A.scal[load];
-  if (S.active == 0) return;
+  if (S.active == 0) {
+    if (blk == 0 && tid == 0) S.step = 0;  // its last step has been taken
+    return;
+  }
   T* out = reinterpret_cast<T*>(A.out) + size_t(load) * 3 * N;
   // boundary rows for the tile above (the first row of tile blockIdx.x + 1, periodic in y)
   T* qb = reinterpret_cast<T*>(A.qb) + size_t(load) * n * ntiles * 3 * n +
@@ -963,6 +967,7 @@ static void set_stencil_smem(int lim) {
   cudaFuncSetAttribute(k_stencil<float, kPCG, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_stencil<double, kPlain, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_stencil<double, kPCG, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(k_stencil<double, kPCG, OCC, double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_stencil<double, kResidual, OCC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_stencil<float, kPCG, OCC, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_stencil<float, kPCG, OCC, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -989,6 +994,7 @@ static void launch_stencil_kernel(int mode, int prec, bool r64, bool planar, dim
     else k_stencil<float, kPCG, OCC><<<grid, block, smem, s>>>(A);
   } else {
     if (mode == kPlain) k_stencil<double, kPlain, OCC><<<grid, block, smem, s>>>(A);
+    else if (mode == kPCG && planar) k_stencil<double, kPCG, OCC, double, true><<<grid, block, smem, s>>>(A);
     else if (mode == kPCG) k_stencil<double, kPCG, OCC><<<grid, block, smem, s>>>(A);
     else k_stencil<double, kResidual, OCC><<<grid, block, smem, s>>>(A);
   }
@@ -1005,9 +1011,9 @@ int launch_stencil(pgj_ctx* c, int mode, int loads, int prec, const void* in, vo
   A.err = c->cond + 2;
   A.rel_flags = rel_flags;
   const size_t tsz = prec == PGJ_FP32 ? 4 : 8;
-  // the FP32 recurrence vectors of a slab-fused context are component-planar, (3, N) per load: the
-  // operator writes its q that way (p is read interleaved)
-  const bool planar = prec == PGJ_FP32 && c->fused && (mode == kPCG || (mode == kPlain && planar_plain));
+  // the recurrence vectors of the plane kernels but p are held by component, (3, N) per load: the operator
+  // writes its q that way (p is read interleaved)
+  const bool planar = c->four && (mode == kPCG || (prec == PGJ_FP32 && mode == kPlain && planar_plain));
   // TMA rows need 16-byte aligned starts and sizes: (3 n * element size) % 16 == 0 and an aligned base
   const size_t rowb = 3 * size_t(n) * tsz;
   A.tma = (rowb % 16 == 0) && (reinterpret_cast<uintptr_t>(in) % 16 == 0) ? 1 : 0;
@@ -1236,21 +1242,6 @@ void element_diagonal(int n, double lam, double mu, double* ed) {
   }
   const double vol8 = 1.0 / (double(n) * n * n) / 8.0;
   for (int i = 0; i < 24; ++i) ed[i] *= vol8;
-}
-
-// s32[c][node] = float(s[3 node + c])
-__global__ void k_scale32(size_t N, const double* __restrict__ s, float* __restrict__ s32) {
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x) {
-    const double a = s[3 * i], b = s[3 * i + 1], c = s[3 * i + 2];
-    s32[i] = float(a);
-    s32[N + i] = float(b);
-    s32[2 * N + i] = float(c);
-  }
-}
-
-int launch_scale32(pgj_ctx* c, cudaStream_t s) {
-  k_scale32<<<296, 256, 0, s>>>(size_t(c->N), c->scale, c->scale32);
-  return check_launch();
 }
 
 int launch_scale(pgj_ctx* c, double alpha, cudaStream_t s) {

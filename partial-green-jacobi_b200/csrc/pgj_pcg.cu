@@ -214,6 +214,7 @@ __global__ void k_init_mask(int loads, LoadScalars* scal, int cap, int* body_run
     LoadScalars& S = scal[l];
     S.active = (S.res2 > S.target2) && (S.iterations < cap) && !S.bad && !S.frozen ? 1 : 0;
     S.failed = 0;
+    S.step = 0;
   }
 }
 
@@ -225,7 +226,7 @@ int launch_init_mask(pgj_ctx* c, int loads, cudaStream_t s) {
 // ------------------------------------------------------------------------------ mixed refinement
 // Start of one refinement sweep, per load: the FP64 certificate decides whether the load still needs
 // a correction; r_in = T(r64), d = 0; the inner target is inner_rtol * ||r64||.
-// `planar`: the FP32 vectors r and d are component-planar, (3, N) per load (slab-fused contexts);
+// `planar`: the FP32 vectors r and d are component-planar, (3, N) per load (plane kernels);
 // the FP64 vectors are node-major interleaved either way.
 __device__ __forceinline__ size_t pidx(size_t node, int c, size_t N, int planar) {
   return planar ? size_t(c) * N + node : 3 * node + c;
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(256) k_inner_start(int n, const double* __rest
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) body_runs[0] = 0;
   const bool done = isfinite(O.absolute) && O.absolute * O.absolute <= O.target2 && !O.bad;
   if (done) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) { S.active = 0; S.touched = 0; S.iterations = 0; }
+    if (blockIdx.x == 0 && threadIdx.x == 0) { S.active = 0; S.touched = 0; S.iterations = 0; S.step = 0; }
     return;
   }
   const size_t off = size_t(load) * N3;
@@ -277,6 +278,7 @@ __global__ void __launch_bounds__(256) k_inner_start(int n, const double* __rest
       S.iterations = 0;
       S.bad = 0;
       S.failed = 0;
+      S.step = 0;
       S.touched = 1;
       S.active = (v[0] > S.target2) && isfinite(v[0]) ? 1 : 0;
     }
@@ -304,14 +306,14 @@ __global__ void __launch_bounds__(256) k_inner_finish(int n, double* __restrict_
 int launch_inner_start(pgj_ctx* c, int loads, double inner_rtol, cudaStream_t s) {
   dim3 grid(2 * 148, loads);
   k_inner_start<float><<<grid, 256, 0, s>>>(c->n, c->r64, static_cast<float*>(c->r), static_cast<float*>(c->d),
-                                            c->scal_out, c->scal_in, c->partials, inner_rtol, c->cond, c->fused);
+                                            c->scal_out, c->scal_in, c->partials, inner_rtol, c->cond, c->four);
   return check_launch();
 }
 
 int launch_inner_finish(pgj_ctx* c, int loads, cudaStream_t s) {
   dim3 grid(2 * 148, loads);
   k_inner_finish<float><<<grid, 256, 0, s>>>(c->n, c->x, static_cast<const float*>(c->d), c->scal_out, c->scal_in,
-                                             c->fused);
+                                             c->four);
   return check_launch();
 }
 
@@ -347,6 +349,7 @@ __global__ void __launch_bounds__(256) k_rel_start(int n, const double* __restri
     S.bad = O.bad;
     S.failed = 0;
     S.reliable = 0;
+    S.step = 0;
     S.active = (O.res2 > O.target2) && (O.iterations < cap) && !O.bad && !O.frozen ? 1 : 0;
   }
 }
@@ -360,10 +363,12 @@ __global__ void k_rel_cond(int loads, const LoadScalars* in, cudaGraphConditiona
   cudaGraphSetConditional(h, any ? 1u : 0u);
 }
 
-// x += d, d = 0 for flagged loads (all loads when `all`)
+// x += d, d = 0 for flagged loads (all loads when `all`); a step alpha p that the plane kernels have not
+// yet added to d goes in with it
 template <typename T>
 __global__ void __launch_bounds__(256) k_rel_fold(int n, double* __restrict__ x, T* __restrict__ d,
-                                                  const LoadScalars* in, LoadScalars* out, int all, int planar) {
+                                                  const T* __restrict__ p, const LoadScalars* in, LoadScalars* out,
+                                                  int all, int planar) {
   const size_t N = size_t(n) * n * n, N3 = 3 * N;
   const int load = blockIdx.y;
   if (!all && !in[load].reliable) return;
@@ -373,14 +378,31 @@ __global__ void __launch_bounds__(256) k_rel_fold(int n, double* __restrict__ x,
     out[load].bad |= in[load].bad;
   }
   const size_t off = size_t(load) * N3;
+  const bool pending = !all && in[load].step;
+  const T alpha = T(in[load].alpha);
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const size_t kt = off + pidx(i, c, N, planar);
-      x[off + 3 * i + c] += double(d[kt]);
+      T v = d[kt];
+      if (pending) v += alpha * p[off + 3 * i + c];
+      x[off + 3 * i + c] += double(v);
       d[kt] = T(0);
     }
   }
+}
+
+// End of an FP64 attempt on the plane kernels: x += d (d by component)
+__global__ void __launch_bounds__(256) k_fold64(int n, double* __restrict__ x, const double* __restrict__ d) {
+  const size_t N = size_t(n) * n * n, off = size_t(blockIdx.y) * 3 * N;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) x[off + 3 * i + c] += d[off + c * N + i];
+}
+
+int launch_fold64(pgj_ctx* c, int loads, cudaStream_t s) {
+  k_fold64<<<dim3(2 * 148, loads), 256, 0, s>>>(c->n, c->x, static_cast<const double*>(c->d));
+  return check_launch();
 }
 
 // flagged loads: r_in = T(r64) (the true residual the FP64 operator just produced); the last block
@@ -446,7 +468,7 @@ int launch_decide(pgj_ctx* c, int loads, cudaGraphConditionalHandle h, cudaStrea
 int launch_rel_start(pgj_ctx* c, int loads, cudaStream_t s) {
   k_rel_start<float><<<dim3(2 * 148, loads), 256, 0, s>>>(c->n, c->r64, static_cast<float*>(c->r),
                                                           static_cast<float*>(c->d), c->scal_out, c->scal_in, c->cap,
-                                                          c->cond, c->fused);
+                                                          c->cond, c->four);
   return check_launch();
 }
 int launch_rel_cond(pgj_ctx* c, int loads, cudaGraphConditionalHandle h, cudaStream_t s) {
@@ -454,13 +476,14 @@ int launch_rel_cond(pgj_ctx* c, int loads, cudaGraphConditionalHandle h, cudaStr
   return check_launch();
 }
 int launch_rel_fold(pgj_ctx* c, int loads, bool all, cudaStream_t s) {
-  k_rel_fold<float><<<dim3(2 * 148, loads), 256, 0, s>>>(c->n, c->x, static_cast<float*>(c->d), c->scal_in,
-                                                         c->scal_out, all ? 1 : 0, c->fused);
+  k_rel_fold<float><<<dim3(2 * 148, loads), 256, 0, s>>>(c->n, c->x, static_cast<float*>(c->d),
+                                                         static_cast<const float*>(c->p), c->scal_in, c->scal_out,
+                                                         all ? 1 : 0, c->four);
   return check_launch();
 }
 int launch_rel_sync(pgj_ctx* c, int loads, cudaStream_t s) {
   k_rel_sync<float><<<dim3(2 * 148, loads), 256, 0, s>>>(c->n, c->r64, static_cast<float*>(c->r), c->scal_out,
-                                                         c->scal_in, c->cap, c->fused);
+                                                         c->scal_in, c->cap, c->four);
   return check_launch();
 }
 

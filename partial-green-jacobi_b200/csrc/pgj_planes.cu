@@ -1,0 +1,142 @@
+// Host side of the plane transform kernels (pgj_planes.cuh): the table of built grids and the launches.
+//
+// Measured, three kernels per iteration (forward / z / inverse), six loads, one B200, us, against the row-packed
+// slab kernels and per-line z passes that these replaced (or, where their slab did not fit, the seven
+// step-by-step kernels): FP64 n = 48 22 / 21 / 25 against 59 / 35 / 33; n = 64 67 / 29 / 69 against
+// 91 / 64 / 50 (the old forward kernel carried the iterate's update, which the inverse one does now);
+// n = 80 118 / 75 / 128 against 254 / 162 / 126; n = 96 188 / 112 / 208 against 1049. FP32 n = 48
+// 19 / 17 / 16 against 40 / 31 / 27; n = 64 26 / 21 / 29 against 47 / 35 / 27; n = 96 88 / 61 / 116 against
+// 178 / 131 / 123; n = 128 212 / 176 / 254 against 1307.
+#include "pgj_planes.cuh"
+#include <cstring>
+#include <mutex>
+#include <set>
+#include <utility>
+
+namespace pgj {
+
+void planes_f64a(PlaneKernels* out, int* count);
+void planes_f64b(PlaneKernels* out, int* count);
+void planes_f64c(PlaneKernels* out, int* count);
+void planes_f32a(PlaneKernels* out, int* count);
+void planes_f32b(PlaneKernels* out, int* count);
+void planes_f32c(PlaneKernels* out, int* count);
+
+namespace {
+constexpr int kMaxPlanes = 64;
+struct Table {
+  PlaneKernels k[kMaxPlanes];
+  int count = 0;
+  Table() {
+    planes_f64a(k, &count);
+    planes_f64b(k, &count);
+    planes_f64c(k, &count);
+    planes_f32a(k, &count);
+    planes_f32b(k, &count);
+    planes_f32c(k, &count);
+  }
+};
+const Table& table() {
+  static const Table t;
+  return t;
+}
+std::mutex g_mutex;
+std::set<std::pair<const void*, int>> g_prepared;  // kernel, device
+}  // namespace
+
+const PlaneKernels* planes_find(int n, int prec) {
+  const Table& t = table();
+  for (int i = 0; i < t.count; ++i)
+    if (t.k[i].n == n && t.k[i].prec == prec) return &t.k[i];
+  return nullptr;
+}
+
+bool fused_selectable(int n, int prec) {
+  const size_t ns = size_t(n / 2 + 1), nsp = ns + (ns & 1);
+  return planes_find(n, prec) && 4 * size_t(n) * nsp * (prec == PGJ_FP32 ? 4 : 8) <= 110 * 1024;
+}
+
+// Shared memory limits of a grid's kernels on the current device.
+int planes_prepare(const PlaneKernels* k) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return set_cuda_error(e);
+  std::lock_guard<std::mutex> lock(g_mutex);
+  const auto key = std::make_pair(k->fwd, device);
+  if (g_prepared.count(key)) return PGJ_OK;
+  e = cudaFuncSetAttribute(k->fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k->inv, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k->z, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->zsmem));
+  if (e != cudaSuccess) return set_cuda_error(e);
+  g_prepared.insert(key);
+  return PGJ_OK;
+}
+
+static PlaneArgs plane_args(pgj_ctx* c, int loads) {
+  const bool f32 = c->prec == PGJ_FP32;
+  PlaneArgs A;
+  std::memset(&A, 0, sizeof(A));
+  A.lpd = c->lpd; A.loads = loads; A.cap = c->cap;
+  A.flex = f32 ? c->flex : 0;
+  A.p = c->p; A.q = c->q; A.d = c->d;
+  A.r = f32 ? c->r : c->sw;  // FP64: c->r holds the certified residual, node-major
+  A.r64 = f32 ? c->r64 : static_cast<const double*>(c->r);
+  A.sp = f32 ? static_cast<const void*>(c->scale32) : static_cast<const void*>(c->scale_pl);
+  A.spec = c->spec; A.shat = c->shat;
+  A.zprev = c->sw;  // FP32 only
+  A.sym = f32 ? static_cast<const void*>(c->symbol32) : static_cast<const void*>(c->symbol);
+  A.tw = f32 ? static_cast<const void*>(static_cast<double2*>(c->tw) + c->n) : c->tw;
+  A.scal = c->scal; A.out = c->scal_out; A.partials = c->partials;
+  A.rel_delta2 = c->rel_delta2; A.counters = c->cond;
+  return A;
+}
+
+static int launch(const void* fn, dim3 grid, int threads, size_t smem, PlaneArgs& A, cudaStream_t s) {
+  void* args[] = {&A};
+  const cudaError_t e = cudaLaunchKernel(fn, grid, dim3(unsigned(threads)), args, smem, s);
+  return e == cudaSuccess ? PGJ_OK : set_cuda_error(e);
+}
+
+static dim3 plane_grid(const pgj_ctx* c, int loads) { return dim3(3, unsigned(c->n / 2), unsigned(loads)); }
+static dim3 line_grid(const PlaneKernels& k, int loads) { return dim3(unsigned((k.m + k.cs - 1) / k.cs), unsigned(loads)); }
+
+int launch_planes_fwd(pgj_ctx* c, int loads, int mode, cudaStream_t s, cudaGraphConditionalHandle hif) {
+  PlaneArgs A = plane_args(c, loads);
+  A.h = hif;
+  A.set_cond = hif ? 1 : 0;
+  A.mode = mode;
+  if (mode == kPlanesUpdate && uses_hf(c, c->prec)) {  // q from the halo-free operator: add its boundary rows
+    A.qb = c->qb;
+    A.hf_ty = c->hg.ty;
+    A.hf_tiles = c->hg.ntiles;
+  }
+  return launch(c->planes->fwd, plane_grid(c, loads), c->planes->nt, c->planes->smem, A, s);
+}
+
+int launch_planes_z(pgj_ctx* c, int loads, bool init, cudaStream_t s) {
+  PlaneArgs A = plane_args(c, loads);
+  A.init = init ? 1 : 0;
+  return launch(c->planes->z, line_grid(*c->planes, loads), c->planes->zt, c->planes->zsmem, A, s);
+}
+
+int launch_planes_inv(pgj_ctx* c, int loads, bool init, cudaStream_t s, cudaGraphConditionalHandle h, bool set_cond) {
+  PlaneArgs A = plane_args(c, loads);
+  A.init = init ? 1 : 0;
+  A.set_cond = set_cond ? 1 : 0;
+  A.h = h;
+  return launch(c->planes->inv, plane_grid(c, loads), c->planes->nt, c->planes->smem, A, s);
+}
+
+// DFT(s) of the designs of `loads` loads, from the scale copy by component.
+int launch_planes_shat(pgj_ctx* c, int loads, cudaStream_t s) {
+  const int designs = (loads + c->lpd - 1) / c->lpd;
+  PlaneArgs A = plane_args(c, loads);
+  A.mode = kPlanesScale;
+  A.spec = c->shat;
+  int st = launch(c->planes->fwd, plane_grid(c, designs), c->planes->nt, c->planes->smem, A, s);
+  if (st) return st;
+  A.forward_only = 1;
+  return launch(c->planes->z, line_grid(*c->planes, designs), c->planes->zt, c->planes->zsmem, A, s);
+}
+
+}  // namespace pgj

@@ -101,14 +101,18 @@ __global__ void k_scale_planes(size_t N, const double* __restrict__ s, T* __rest
   }
 }
 
+int launch_scale_planes(pgj_ctx* c, int loads, cudaStream_t s) {
+  const size_t N = size_t(c->N);
+  const dim3 grid(unsigned((N + 255) / 256 < 148 ? (N + 255) / 256 : 148), unsigned((loads + c->lpd - 1) / c->lpd));
+  if (c->prec == PGJ_FP32) k_scale_planes<float><<<grid, 256, 0, s>>>(N, c->scale, c->scale32);
+  else k_scale_planes<double><<<grid, 256, 0, s>>>(N, c->scale, c->scale_pl);
+  return check_launch();
+}
+
 int launch_resident(pgj_ctx* c, int loads, cudaStream_t s) {
   const ResidentKernel& k = *c->res;
   const bool f32 = c->prec == PGJ_FP32;
-  const size_t N = size_t(c->N);
-  const dim3 grid(unsigned((N + 255) / 256 < 148 ? (N + 255) / 256 : 148), unsigned((loads + c->lpd - 1) / c->lpd));
-  if (f32) k_scale_planes<float><<<grid, 256, 0, s>>>(N, c->scale, c->scale32);
-  else k_scale_planes<double><<<grid, 256, 0, s>>>(N, c->scale, c->scale_pl);
-  int st = check_launch();
+  int st = launch_scale_planes(c, loads, s);
   if (st) return st;
   ResidentArgs A;
   A.lpd = c->lpd; A.cap = c->cap; A.loads = loads;
@@ -120,9 +124,8 @@ int launch_resident(pgj_ctx* c, int loads, cudaStream_t s) {
     A.sp = c->scale32; A.sym = c->symbol32; A.tw = static_cast<double2*>(c->tw) + c->n;
     A.r0 = c->r64; A.r = c->r; A.d = c->d; A.p = c->p;
   } else {
-    // the certified residual's buffer becomes the correction, p and s.w buffers hold r and p
     A.sp = c->scale_pl; A.sym = c->symbol; A.tw = c->tw;
-    A.r0 = static_cast<const double*>(c->r); A.r = c->p; A.d = c->r; A.p = c->sw;
+    A.r0 = static_cast<const double*>(c->r); A.r = c->sw; A.d = c->d; A.p = c->p;
   }
   cudaLaunchAttribute at;
   const cudaLaunchConfig_t cfg = config(k, loads, &at, s);

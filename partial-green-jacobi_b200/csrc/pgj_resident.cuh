@@ -24,9 +24,10 @@
 // What bounds it: below n = 24 the four exchanges (0.8k to 2.5k clocks each: block sum, travel, and for the
 // two that order the spectra a release that waits for the block's stores), above that the element
 // arithmetic and the latency of the phases' loads at 9 to 16 warps per SM. Per iteration, six loads, one
-// B200, against the four separate kernels (FP64 / mixed): n = 16 10.6 / 9.8 us against 43.8 / 51.3,
-// n = 24 21.1 / 18.3 against 51.9 / 56.3, n = 32 29.4 / 23.9 against 63.1 / 63.7, n = 36 68 / 48 against
-// 96 / 87, n = 48 130 / 88 against 154 / 131. FP64 at n = 40 was slower (100 against 93) and is not built.
+// B200, against separate kernels (pgj_planes.cuh; FP64 / mixed): n = 16 10.6 / 9.8 us against 38.6 / 47.8,
+// n = 24 21.1 / 18.3, n = 32 29.4 / 23.9, n = 36 68 / 48 against 65 / 65, n = 40 100 / 65 against 71 / 69,
+// n = 48 130 / 88 against 102 / 87: above n = 32 in FP64 and n = 36 in mixed precision, where p or q no longer
+// fit in shared memory, the whole GPU's separate kernels win and these are not built.
 //
 // Vectors are held plane by plane, [z][component][y][x] per load; p is [z][y][x][component], the
 // order in which the operator reads whole triples. The blocks of a cluster always take the same
@@ -48,7 +49,7 @@ struct ResidentArgs {
   double* x;              // (L, 3N) FP64 iterate
   const double* r0;       // (L, 3N) certified residual
   void* r;                // (L, 3N) T recurrence residual
-  void* d;                // (L, 3N) T correction; FP64: may be r0 (read before it is written)
+  void* d;                // (L, 3N) T correction
   void* p;                // (L, 3N) T direction where it does not fit in shared memory
   void* q;                // (L, 3N) T
   void* spec;             // (L, 3, n, n ns) complex T
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(Cfg::NT, 1) k_resident_pcg(const ResidentArgs 
   const T* sym = static_cast<const T*>(A.sym);
 
   for (int i = tid; i < N; i += NT) tw[i] = static_cast<const C*>(A.tw)[i];
-  // r = T(certified residual), plane by plane through shared memory: d may be the same memory
+  // r = T(certified residual), plane by plane through shared memory
   {
     T* st = reinterpret_cast<T*>(buf);
     constexpr int PB = int((Cfg::smem - Cfg::o_u) / (PL * sizeof(T)));  // planes staged at a time

@@ -1,4 +1,4 @@
-// Cluster-resident PCG kernels, FP32 recurrences, grids from 30 (shapes: pgj_resident.cuh).
+// Cluster-resident PCG kernels, FP32 recurrences, grids 30 to 36 (shapes: pgj_resident.cuh).
 #include "pgj_resident.cuh"
 
 namespace pgj {
@@ -7,7 +7,5 @@ void resident_f32b(ResidentKernel* out, int* count) {
   out[(*count)++] = resident_entry<ResidentCfg<30, float, 15, 10, 320, 3, 32, true, true, true>>();
   out[(*count)++] = resident_entry<ResidentCfg<32, float, 16, 8, 384, 3, 34, true, true, true>>();
   out[(*count)++] = resident_entry<ResidentCfg<36, float, 12, 6, 384, 5, 57, true, true, false>>();
-  out[(*count)++] = resident_entry<ResidentCfg<40, float, 10, 8, 384, 6, 84, true, false, false>>();
-  out[(*count)++] = resident_entry<ResidentCfg<48, float, 16, 8, 384, 5, 75, false, true, false>>();
 }
 }  // namespace pgj

@@ -232,7 +232,7 @@ class Operator:
         nbytes = (C.c_double * 8)()
         _lib.check(_lib.lib().pgj_profile_iteration(self._ctx, m.shape[0], m.ctypes.data, int(reps), ms, nbytes,
                                                     _stream_ptr()), "pgj_profile_iteration")
-        if self.fused_iteration:
+        if all(m == 0.0 for m in ms[4:8]):
             names = ["operator", "update_fft_xy", "fft_z_symbol", "ifft_xy_update_p"]
         else:
             names = ["operator", "update_ur", "fft_x", "fft_y", "fft_z_symbol", "ifft_y", "ifft_x", "update_p"]
