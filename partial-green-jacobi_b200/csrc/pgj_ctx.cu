@@ -88,8 +88,6 @@ static Layout make_layout(int n, int D, int lpd, int prec) {
   y.spec = take(2 * tsz * 3 * size_t(n) * n * nsp * L);
   y.shat = take(2 * tsz * 3 * size_t(n) * n * nsp * D);
   y.scale32 = take(prec == PGJ_FP32 ? sizeof(float) * N3 * D : 0);
-  // boundary rows of the halo-free FP32 operator: n planes x n / ty tiles x 3n per load, ty >= 2
-  y.qb = take(prec == PGJ_FP32 && n == 64 ? sizeof(float) * (N3 / 2 + 3 * size_t(n)) * L : 0);
   const size_t halo = resident_halo_bytes(n, prec);
   y.scale_pl = take(prec == PGJ_FP64 && planes_find(n, prec) ? sizeof(double) * N3 * D : 0);
   y.halo = take(halo * L);
@@ -434,7 +432,8 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
   c->N = (long long)n * n * n; c->ns = n / 2 + 1; c->Nh = (long long)n * n * c->ns;
   c->kc = make_opconst(n, lam, mu);
   make_fft_plan(n, &c->plan);
-  c->sg = stencil_geom(n, loads);
+  c->geo64 = rows_geom(n, loads, true);
+  c->geo32 = rows_geom(n, loads, false);
   c->fg = fft_geom(n, precision == PGJ_FP32 ? 4 : 8, c->plan);
   c->lay = y;
   c->base = static_cast<char*>(workspace);
@@ -450,12 +449,6 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
   c->x = reinterpret_cast<double*>(b + y.x);
   c->r64 = precision == PGJ_FP32 ? reinterpret_cast<double*>(b + y.r64) : nullptr;
   c->r = b + y.r; c->p = b + y.p; c->q = b + y.q; c->sw = b + y.sw; c->spec = b + y.spec;
-  c->qb = precision == PGJ_FP32 && n == 64 ? static_cast<void*>(b + y.qb) : nullptr;
-  c->hg = hf_geom(n, loads);
-  {
-    const char* e = std::getenv("PGJ_HF");
-    c->hf = c->qb != nullptr && !(e && e[0] == '0') ? 1 : 0;
-  }
   c->shat = b + y.shat;
   c->scale_pl = reinterpret_cast<double*>(b + y.scale_pl);
   c->halo = b + y.halo;
@@ -482,7 +475,7 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
   cudaError_t e = cudaMemsetAsync(workspace, 0, y.total, s);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->graphs->cap, cudaStreamNonBlocking);
   if (e != cudaSuccess) st = set_cuda_error(e);
-  if (!st) st = prepare_stencil_kernels();
+  if (!st) st = prepare_rows();
   if (!st) st = prepare_fft_kernels();
   if (!st && c->planes) st = planes_prepare(c->planes);
   c->four = c->planes && !std::getenv("PGJ_UNFUSED") ? 1 : 0;
@@ -502,7 +495,6 @@ int pgj_ctx_create_batch(int n, int designs, int loads, int precision, double la
     DesignScope view(c, d);
     st = launch_scale(c, 0.0, s);  // scale = 1 until an alpha is selected
   }
-  if (!st) st = autotune_stencil(c, s);
   if (!st) st = autotune_fft(c, s);
   if (st) {
     delete c->graphs;
@@ -808,14 +800,16 @@ int pgj_fused_iteration(pgj_ctx* c) { return c ? c->fused : -1; }
 
 int pgj_tile_shapes(pgj_ctx* c, int* out) {
   if (!c || !out) return PGJ_ERR_ARGUMENT;
-  out[0] = c->sg.ty; out[1] = c->sg.zc; out[2] = c->fg.rb; out[3] = c->fg.kcy; out[4] = c->fg.kcz;
+  const StencilGeom& g = c->prec == PGJ_FP32 ? c->geo32 : c->geo64;
+  out[0] = g.ty; out[1] = g.zc; out[2] = c->fg.rb; out[3] = c->fg.kcy; out[4] = c->fg.kcz;
   out[5] = c->fused;
   return PGJ_OK;
 }
 
 int pgj_tile_config(pgj_ctx* c, int* out) {
   if (!c || !out) return PGJ_ERR_ARGUMENT;
-  out[0] = c->sg.ty; out[1] = c->sg.zc; out[2] = c->sg.stages; out[3] = c->sg.occ;
+  const StencilGeom& g = c->prec == PGJ_FP32 ? c->geo32 : c->geo64;
+  out[0] = g.ty; out[1] = g.zc; out[2] = 0; out[3] = g.occ;
   out[4] = c->fft_req[0]; out[5] = c->fft_req[1]; out[6] = c->fft_req[2];
   out[7] = c->fused; out[8] = c->tile_source;
   return PGJ_OK;

@@ -486,19 +486,26 @@ int autotune_fft(pgj_ctx* c, cudaStream_t s) {
     if (it != g_fft_tuned.end()) {
       c->fg = it->second.first;
       for (int k = 0; k < 3; ++k) c->fft_req[k] = it->second.second[k];
+      TileEntry t;
+      c->tile_source = tile_table(c->n, c->prec, &t) ? 1 : 0;
       return PGJ_OK;
     }
   }
-  if (std::getenv("PGJ_FFT_RB") || std::getenv("PGJ_FFT_NKY") || std::getenv("PGJ_FFT_NKZ")) return PGJ_OK;
+  if (std::getenv("PGJ_FFT_RB") || std::getenv("PGJ_FFT_NKY") || std::getenv("PGJ_FFT_NKZ")) {
+    c->tile_source = 2;
+    return PGJ_OK;
+  }
   const int eb = c->prec == PGJ_FP32 ? 4 : 8;
   TileEntry t;
   if (tile_table(c->n, c->prec, &t)) {
+    c->tile_source = 1;
     c->fg = fft_geom(c->n, eb, c->plan, t.rb, t.nky, t.nkz);
     c->fft_req[0] = t.rb; c->fft_req[1] = t.nky; c->fft_req[2] = t.nkz;
     std::lock_guard<std::mutex> lock(g_fft_mutex);
     g_fft_tuned[key] = {c->fg, {t.rb, t.nky, t.nkz}};
     return PGJ_OK;
   }
+  c->tile_source = 0;
   std::vector<FFTGeom> cands;
   std::vector<std::array<int, 3>> reqs;
   for (int rb : {8, 16})

@@ -16,17 +16,16 @@ struct FFTPlan {
 };
 bool make_fft_plan(int n, FFTPlan* plan);
 
-// Launch geometry of the streaming stencil for a grid edge n.
+// Launch geometry of the operator for a grid edge n (rows_geom).
 struct StencilGeom {
-  int ty;      // output node rows per block (block is n x (ty+1) threads)
+  int ty;      // output node rows per block (block is n / 2 x (ty + 1) threads)
   int ntiles;  // tiles along y
   int zc;      // output node planes per block
   int nchunks; // chunks along z
-  int stages;  // node-plane buffers of the TMA staging pipeline (2..4)
-  int occ;     // 1: up to 512 threads per block; 3: at most 256 threads, three blocks per SM
+  int occ;     // blocks per SM
 };
-StencilGeom stencil_geom(int n, int loads);
-StencilGeom stencil_geom_shape(int n, int ty, int zc, int stages = 2, int occ = 1);
+// `wide`: FP64 arithmetic
+StencilGeom rows_geom(int n, int lpd, bool wide);
 
 // Geometry of the FFT passes.
 struct FFTGeom {
@@ -55,11 +54,6 @@ struct StencilArgs {
   LoadScalars* scal;           // pcg / residual modes
   double* partials;            // [load][4][nblk]
   OpConst kc;
-  int iteration_cap;
-  int tma;                     // stage planes with bulk async copies (aligned rows) instead of cp.async
-  int stages;                  // plane buffers in the staging pipeline
-  int* err;                    // set to 1 if a bounded device wait expired
-  void* qb;                    // halo-free recurrence operator: boundary rows (L, n, ntiles, 3, n)
 };
 
 // Partial-sum slots per load per kernel (blocks per load upper bound).
@@ -73,7 +67,7 @@ constexpr int kAuxDoubles = kAuxPartials + kMaxPartials;
 
 struct Layout {
   size_t a, scale, scale32, symbol, symbol32, tw, solutions, f, x, r, p, q, sw, spec, shat, partials, scal, macros,
-      cond, r64, d, aux, qb, scale_pl, halo, total;
+      cond, r64, d, aux, scale_pl, halo, total;
 };
 
 struct Graphs;
@@ -91,7 +85,7 @@ struct pgj_ctx {
   long long Nh;
   pgj::OpConst kc;
   pgj::FFTPlan plan;
-  pgj::StencilGeom sg;
+  pgj::StencilGeom geo64, geo32;  // the operator's launches in FP64 and FP32 arithmetic
   pgj::FFTGeom fg;
   pgj::Layout lay;
   char* base;
@@ -109,9 +103,6 @@ struct pgj_ctx {
   void* r;             // (L, 3N) T
   void* p;             // (L, 3N) T
   void* q;             // (L, 3N) T
-  void* qb;            // FP32 contexts at n = 64: (L, n, n / hg.ty, 3, n) boundary rows of the halo-free operator
-  pgj::StencilGeom hg; // halo-free recurrence operator geometry (FP32 slab-fused contexts)
-  int hf;              // FP32 slab-fused recurrences use the halo-free operator (PGJ_HF=0: the halo form)
   void* sw;            // (L, 3N) T  s . w (unprojected preconditioned residual); plane kernels in FP64: the residual
   void* spec;          // (L, 3, n, n, nsp) complex T (plane kernels: rows of ns)
   void* shat;          // (D, 3, n, n, nsp) complex T: DFT of each component of the scale field
@@ -136,8 +127,8 @@ struct pgj_ctx {
   int mixed_mode;      // 0 reliable-update CG, 1 restarted refinement sweeps
   int op64;            // FP32 contexts: the recurrence operator computes in FP64 (FP32 vectors)
   int cap;             // per-load PCG iteration cap (4000, the reference's, unless set)
-  int flex;            // FP32 slab-fused recurrences: flexible (Polak-Ribiere) beta
-  int tile_source;     // 0 tuned by timing at creation, 1 tile table, 2 environment override
+  int flex;            // FP32 recurrences on the plane kernels: flexible (Polak-Ribiere) beta
+  int tile_source;     // FFT tiles: 0 tuned by timing at creation, 1 tile table, 2 environment override
   int fft_req[3];      // requested FFT tiles (rows per x block, y chunks, z chunks)
   int last_refinements;
   int pending_loads;       // loads of the solve enqueued by pgj_solve_async
@@ -150,14 +141,15 @@ struct pgj_ctx {
 };
 
 namespace pgj {
-// operator (pgj_operator.cu)
-// planar_plain: plain mode writing q component-planar, as the recurrence operator of an FP32
-// context does (the tuner)
+// operator (pgj_rows.cu)
 int launch_stencil(pgj_ctx* c, int mode, int loads, int prec, const void* in, void* out, const double* f,
-                   const int32_t* active_ext, cudaStream_t s, const LoadScalars* rel_flags = nullptr,
-                   bool planar_plain = false);
-// offline-tuned tile shapes per (n, precision)
-struct TileEntry { int n, prec, ty, zc, stages, occ, rb, nky, nkz; };
+                   const int32_t* active_ext, cudaStream_t s, const LoadScalars* rel_flags = nullptr);
+// the recurrence operator q = K p (and alpha = r.z / p.q) of one PCG iteration
+inline int launch_recurrence_operator(pgj_ctx* c, int loads, int prec, cudaStream_t s) {
+  return launch_stencil(c, kPCG, loads, prec, c->p, c->q, nullptr, nullptr, s);
+}
+// offline-tuned tile shapes per (n, precision); right-hand side, scale, norms (pgj_operator.cu)
+struct TileEntry { int n, prec, rb, nky, nkz; };
 bool tile_table(int n, int prec, TileEntry* out);
 int launch_rhs(pgj_ctx* c, int loads, const double* macros_dev, double* f, cudaStream_t s);
 int launch_scale(pgj_ctx* c, double alpha, cudaStream_t s);
@@ -186,13 +178,6 @@ int launch_planes_inv(pgj_ctx* c, int loads, bool init, cudaStream_t s, cudaGrap
 int launch_planes_shat(pgj_ctx* c, int loads, cudaStream_t s);
 // copies the scale fields of the loads' designs by component, in the context precision (pgj_resident.cu)
 int launch_scale_planes(pgj_ctx* c, int loads, cudaStream_t s);
-// halo-free FP32 recurrence operator (pgj_operator.cu): geometry, launch, and whether a context's
-// recurrence uses it (FP32, plane kernels, FP32 arithmetic, not switched off)
-StencilGeom hf_geom(int n, int lpd);
-int launch_stencil_hf(pgj_ctx* c, int loads, cudaStream_t s);
-inline bool uses_hf(const pgj_ctx* c, int prec) { return prec == PGJ_FP32 && c->four && c->hf && !c->op64; }
-// the recurrence operator q = K p (and alpha = r.z / p.q) of one PCG iteration
-int launch_recurrence_operator(pgj_ctx* c, int loads, int prec, cudaStream_t s);
 // cluster-resident PCG (pgj_resident.cu): a whole attempt's recurrence in one launch
 const ResidentKernel* resident_prepare(int n, int prec);
 size_t resident_halo_bytes(int n, int prec);
@@ -234,10 +219,8 @@ struct DesignScope {
 
 int set_cuda_error(cudaError_t e);
 // one-time kernel attributes (dynamic shared memory limits); called at context creation
-int prepare_stencil_kernels();
+int prepare_rows();
 int launch_wait_selftest(int tries, int* flag, cudaStream_t s);
-// times candidate tile shapes of the operator on the context's buffers and keeps the fastest
-int autotune_stencil(pgj_ctx* c, cudaStream_t s);
 // times candidate tile shapes of the Green passes and keeps the fastest
 int autotune_fft(pgj_ctx* c, cudaStream_t s);
 int prepare_fft_kernels();

@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(256) k_rel_fold(int n, double* __restrict__ x,
     for (int c = 0; c < 3; ++c) {
       const size_t kt = off + pidx(i, c, N, planar);
       T v = d[kt];
-      if (pending) v += alpha * p[off + 3 * i + c];
+      if (pending) v += alpha * p[kt];
       x[off + 3 * i + c] += double(v);
       d[kt] = T(0);
     }

@@ -105,11 +105,6 @@ int launch_planes_fwd(pgj_ctx* c, int loads, int mode, cudaStream_t s, cudaGraph
   A.h = hif;
   A.set_cond = hif ? 1 : 0;
   A.mode = mode;
-  if (mode == kPlanesUpdate && uses_hf(c, c->prec)) {  // q from the halo-free operator: add its boundary rows
-    A.qb = c->qb;
-    A.hf_ty = c->hg.ty;
-    A.hf_tiles = c->hg.ntiles;
-  }
   return launch(c->planes->fwd, plane_grid(c, loads), c->planes->nt, c->planes->smem, A, s);
 }
 

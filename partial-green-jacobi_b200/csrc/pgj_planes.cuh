@@ -16,7 +16,7 @@
 // packing of rows and no pass for the split. The half spectrum is (component, z, m) with m = ky ns + kx:
 // the z kernel reads CS columns m of every plane as one contiguous run. The correction d takes its step
 // in the inverse kernel, which reads p anyway (LoadScalars::step marks a load whose step is pending).
-// Everything but p is held by component, (3, N) per load, and moves two values at a time.
+// Vectors are held by component, (3, N) per load, and move two values at a time.
 //
 // Bounds: each kernel moves its operands once; the x/y kernels are limited by the loads in flight that
 // their planes leave room for (registers and shared memory), the z kernel by the same and, in FP64, by
@@ -31,7 +31,7 @@ enum PlaneMode { kPlaneUpdate = 0, kPlaneInit = 1, kPlaneSync = 2, kPlaneScale =
 
 struct PlaneArgs {
   int lpd, loads, cap, mode, flex, init, set_cond, forward_only;
-  void* p;                // (L, 3N) T directions, node-major
+  void* p;                // (L, 3, N) T directions
   const void* q;          // (L, 3, N) T K p
   void* r;                // (L, 3, N) T residual
   void* d;                // (L, 3, N) T correction
@@ -42,8 +42,6 @@ struct PlaneArgs {
   void* zprev;            // flexible beta: (L, 3, N) T z of the previous direction
   const void* sym;        // (6, n, n ns) T
   const void* tw;         // n complex T
-  const void* qb;         // halo-free operator: rows (L, n, tiles, 3, n) missing from the first row of a tile
-  int hf_ty, hf_tiles;    // its tile rows (0: q is complete) and tiles
   LoadScalars* scal;
   const LoadScalars* out; // sync: certificate records
   double* partials;
@@ -132,8 +130,6 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
   if (mode == kPlaneUpdate) {
     const C* q2 = reinterpret_cast<const C*>(static_cast<const T*>(A.q) + off);
     const T al = T(S.alpha);
-    const int ty = A.hf_ty;
-    const T* qb = ty ? static_cast<const T*>(A.qb) + ((size_t(load) * N + z) * A.hf_tiles * 3 + c) * N : nullptr;
     const C* zp = A.flex ? reinterpret_cast<const C*>(static_cast<const T*>(A.zprev) + off) : nullptr;
 #pragma unroll 1
     for (int e0 = tid; e0 < H; e0 += UNR * NT) {
@@ -150,15 +146,6 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
       for (int u = 0; u < UNR; ++u) {
         const int e = e0 + u * NT, y = e / (N / 2), x = 2 * (e - y * (N / 2));
         if (e >= H) continue;
-        if (ty) {
-          const int t = y / ty;
-          if (t * ty == y) {  // first row of an operator tile
-            const C ba = *reinterpret_cast<const C*>(qb + size_t(t) * 3 * N + x);
-            const C bb = *reinterpret_cast<const C*>(qb + (size_t(A.hf_tiles) + t) * 3 * N + x);
-            qa[u].x += ba.x; qa[u].y += ba.y;
-            qv[u].x += bb.x; qv[u].y += bb.y;
-          }
-        }
         C a, b;
         a.x = ra[u].x - al * qa[u].x; a.y = ra[u].y - al * qa[u].y;
         b.x = rb[u].x - al * qv[u].x; b.y = rb[u].y - al * qv[u].y;
@@ -420,15 +407,13 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_inv(const __grid_
   if (!step && !active) return;
   const size_t off = size_t(load) * N3 + size_t(c) * NV + size_t(z) * NN;
   C* d2 = reinterpret_cast<C*>(static_cast<T*>(A.d) + off);
-  T* p = static_cast<T*>(A.p) + size_t(load) * N3 + 3 * (size_t(z) * NN) + c;
+  C* p2 = reinterpret_cast<C*>(static_cast<T*>(A.p) + off);
   const T al = T(S.alpha);
   if (!active) {  // the load stopped with this step
     for (int e = tid; e < H; e += NT) {
-      const T* pa = p + 6 * size_t(e);
-      const T* pb = pa + 3 * size_t(NN);
-      const C da = d2[e], db = d2[H + e];
-      d2[e] = cmk<C>(da.x + al * pa[0], da.y + al * pa[3]);
-      d2[H + e] = cmk<C>(db.x + al * pb[0], db.y + al * pb[3]);
+      const C da = d2[e], db = d2[H + e], pa = p2[e], pb = p2[H + e];
+      d2[e] = cmk<C>(da.x + al * pa.x, da.y + al * pa.y);
+      d2[H + e] = cmk<C>(db.x + al * pb.x, db.y + al * pb.y);
     }
     return;
   }
@@ -472,20 +457,14 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_inv(const __grid_
   constexpr int UNR = sizeof(T) == 4 ? 2 : 1;
 #pragma unroll 1
   for (int e0 = tid; e0 < H; e0 += UNR * NT) {
-    C sa[UNR], sb[UNR], da[UNR], db[UNR];
-    T pv[UNR][4];
+    C sa[UNR], sb[UNR], da[UNR], db[UNR], pa[UNR], pb[UNR];
 #pragma unroll
     for (int u = 0; u < UNR; ++u) {
       const int e = e0 + u * NT;
       if (e >= H) continue;
-      const T* pa = p + 6 * size_t(e);
-      const T* pb = pa + 3 * size_t(NN);
       sa[u] = __ldg(s2 + e); sb[u] = __ldg(s2 + H + e);
-      if (init) {
-        pv[u][0] = pv[u][1] = pv[u][2] = pv[u][3] = T(0);
-      } else {
-        pv[u][0] = pa[0]; pv[u][1] = pa[3]; pv[u][2] = pb[0]; pv[u][3] = pb[3];
-      }
+      pa[u] = pb[u] = cmk<C>(T(0), T(0));
+      if (!init) { pa[u] = p2[e]; pb[u] = p2[H + e]; }
       if (step) { da[u] = d2[e]; db[u] = d2[H + e]; }
     }
 #pragma unroll
@@ -493,20 +472,16 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_inv(const __grid_
       const int e = e0 + u * NT, y = e / (N / 2), x = 2 * (e - y * (N / 2));
       if (e >= H) continue;
       if (step) {
-        d2[e] = cmk<C>(da[u].x + al * pv[u][0], da[u].y + al * pv[u][1]);
-        d2[H + e] = cmk<C>(db[u].x + al * pv[u][2], db[u].y + al * pv[u][3]);
+        d2[e] = cmk<C>(da[u].x + al * pa[u].x, da[u].y + al * pa[u].y);
+        d2[H + e] = cmk<C>(db[u].x + al * pb[u].x, db[u].y + al * pb[u].y);
       }
       const C w0 = buf[y * PX + x], w1 = buf[y * PX + x + 1];
-      const T z0 = sa[u].x * w0.x - m, z1 = sa[u].y * w1.x - m, z2 = sb[u].x * w0.y - m, z3 = sb[u].y * w1.y - m;
-      T* pa = p + 6 * size_t(e);
-      T* pb = pa + 3 * size_t(NN);
-      pa[0] = z0 + beta * pv[u][0];
-      pa[3] = z1 + beta * pv[u][1];
-      pb[0] = z2 + beta * pv[u][2];
-      pb[3] = z3 + beta * pv[u][3];
+      const C za = cmk<C>(sa[u].x * w0.x - m, sa[u].y * w1.x - m), zb = cmk<C>(sb[u].x * w0.y - m, sb[u].y * w1.y - m);
+      p2[e] = cmk<C>(za.x + beta * pa[u].x, za.y + beta * pa[u].y);
+      p2[H + e] = cmk<C>(zb.x + beta * pb[u].x, zb.y + beta * pb[u].y);
       if (zp) {
-        zp[e] = cmk<C>(z0, z1);
-        zp[H + e] = cmk<C>(z2, z3);
+        zp[e] = za;
+        zp[H + e] = zb;
       }
     }
   }
