@@ -130,17 +130,19 @@ static int capture_iteration(pgj_ctx* c, int L, cudaStream_t s, cudaGraphConditi
 // kernels, which first refresh the scale copies and DFT(s) in case the scale was rewritten through its view.
 static long long first_direction_launches(const pgj_ctx* c) { return c->four ? 3 + 3 : 6; }
 
-static int capture_first_direction(pgj_ctx* c, int L, cudaStream_t s) {
+// A handle `h` is set to whether any load is active: a conditional's default applies once per graph launch, so
+// the loop of a second attempt within a launch would not run without it.
+static int capture_first_direction(pgj_ctx* c, int L, cudaStream_t s, cudaGraphConditionalHandle h = 0) {
   int st;
   if (c->four) {
     if ((st = launch_scale_planes(c, L, s))) return st;
     if ((st = launch_planes_shat(c, L, s))) return st;
     if ((st = launch_planes_fwd(c, L, kPlanesInit, s))) return st;
     if ((st = launch_planes_z(c, L, true, s))) return st;
-    return launch_planes_inv(c, L, true, s, 0, false);
+    return launch_planes_inv(c, L, true, s, h, h != 0);
   }
   st = launch_green(c, L, c->prec, c->r, true, s);
-  return st ? st : launch_update_p(c, L, c->prec, true, s, 0, false);
+  return st ? st : launch_update_p(c, L, c->prec, true, s, h, h != 0);
 }
 
 // Appends a conditional node of `type` after the current capture point of `s` and returns its body
@@ -238,38 +240,15 @@ static int end_capture(cudaStream_t s, cudaGraph_t* g, int st) {
 
 // Appends to the capture on `s`: directions init, then WHILE(any load active){iteration}.
 static int capture_pcg(pgj_ctx* c, int L, cudaStream_t s, bool reliable = false) {
-  int st = capture_first_direction(c, L, s);
-  if (st) return st;
-  cudaStreamCaptureStatus cs;
-  cudaGraph_t cg = nullptr;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t ndeps = 0;
-  cudaError_t e = cudaStreamGetCaptureInfo(s, &cs, nullptr, &cg, &deps, &ndeps);
   cudaGraphConditionalHandle h = 0;
-  if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, cg, 1, cudaGraphCondAssignDefault);
-  cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-  cp.conditional.handle = h;
-  cp.conditional.type = cudaGraphCondTypeWhile;
-  cp.conditional.size = 1;
-  cudaGraphNode_t node = nullptr;
-  if (e == cudaSuccess) e = cudaGraphAddNode(&node, cg, deps, ndeps, &cp);
-  if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(s, &node, 1, cudaStreamSetCaptureDependencies);
-  if (e != cudaSuccess) return set_cuda_error(e);
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  cudaStream_t s2;
-  e = cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking);
-  if (e != cudaSuccess) return set_cuda_error(e);
-  e = cudaStreamBeginCaptureToGraph(s2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) {
-    st = set_cuda_error(e);
-  } else {
-    st = reliable ? capture_iteration_rel(c, L, s2, h) : capture_iteration(c, L, s2, h, true);
-    cudaGraph_t bg = body;
-    cudaError_t e2 = cudaStreamEndCapture(s2, &bg);
-    if (!st && e2 != cudaSuccess) st = set_cuda_error(e2);
-  }
-  cudaStreamDestroy(s2);
-  return st;
+  cudaGraph_t body = nullptr;
+  int st = make_handle(s, &h, 1);
+  if (!st) st = capture_first_direction(c, L, s, h);
+  if (!st) st = add_conditional(s, &h, 1, cudaGraphCondTypeWhile, &body);
+  if (st) return st;
+  return capture_into(body, [&](cudaStream_t s2) {
+    return reliable ? capture_iteration_rel(c, L, s2, h) : capture_iteration(c, L, s2, h, true);
+  });
 }
 
 // One attempt: FP64 -> init masks, PCG loop, certify; mixed reliable -> FP32 recurrence with

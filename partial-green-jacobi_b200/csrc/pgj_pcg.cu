@@ -166,10 +166,14 @@ __global__ void __launch_bounds__(256) k_update_p(int n, int loads, T* __restric
   if (set_cond && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
     int any = 0;
     for (int l = 0; l < loads; ++l) any |= scal[l].active;
-    const int runs = ++body_runs[0];
-    body_runs[5] += 1;                             // loop bodies over the whole solve (launch accounting)
-    if (runs >= bound) body_runs[1] = 1;  // recorded: loop stopped by the bound
-    cudaGraphSetConditional(h, (any && runs < bound) ? 1u : 0u);
+    if (init) {
+      cudaGraphSetConditional(h, any ? 1u : 0u);  // the attempt's loop, which the last attempt left at 0
+    } else {
+      const int runs = ++body_runs[0];
+      body_runs[5] += 1;                    // loop bodies over the whole solve (launch accounting)
+      if (runs >= bound) body_runs[1] = 1;  // recorded: loop stopped by the bound
+      cudaGraphSetConditional(h, (any && runs < bound) ? 1u : 0u);
+    }
   }
   const LoadScalars& S = scal[load];
   if (!S.active) return;

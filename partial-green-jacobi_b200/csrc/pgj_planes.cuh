@@ -397,10 +397,14 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_inv(const __grid_
   if (A.set_cond && c == 0 && z == 0 && load == 0 && tid == 0) {
     int any = 0;
     for (int l = 0; l < A.loads; ++l) any |= A.scal[l].active;
-    const int runs = ++A.counters[0];
-    A.counters[5] += 1;                          // loop bodies over the whole solve
-    if (runs >= A.cap + 100) A.counters[1] = 1;  // recorded: loop stopped by the bound
-    cudaGraphSetConditional(A.h, (any && runs < A.cap + 100) ? 1u : 0u);
+    if (A.init) {
+      cudaGraphSetConditional(A.h, any ? 1u : 0u);  // the attempt's loop, which the last attempt left at 0
+    } else {
+      const int runs = ++A.counters[0];
+      A.counters[5] += 1;                          // loop bodies over the whole solve
+      if (runs >= A.cap + 100) A.counters[1] = 1;  // recorded: loop stopped by the bound
+      cudaGraphSetConditional(A.h, (any && runs < A.cap + 100) ? 1u : 0u);
+    }
   }
   const LoadScalars& S = A.scal[load];
   const bool step = S.step != 0, active = S.active != 0;
