@@ -3,7 +3,7 @@
 // For v_l = u_l + A_l on an element (A_l the affine field of the macro strain), the element
 // energy v_i^T Ke v_j equals sum_m Q_i[m] . P_j[m] in the modal basis (the Hadamard transform is
 // orthogonal up to the same factor on both sides), with P_j the modal element action for a = 1.
-// One pass over the elements therefore gives every pair (i <= j) at once:
+// One pass over the elements therefore gives every pair at once:
 //   e_l(el)  = v_l^T Ke v_l / h^3                      (energy.cu:7-24 in exp/asg_scenarios_20261105)
 //   C_ij     = mean_el( a v_i^T Ke v_j ) / h^3          (polarisation in reproduction.py:166-176)
 #include "pgj_internal.h"
@@ -12,6 +12,7 @@ namespace pgj {
 
 struct EnergyArgs {
   int n, loads;
+  int zc;                // element planes per block
   const double* u;       // (loads, 3N)
   const double* macros;  // (loads, 6) device
   const double* a;       // (N)
@@ -22,111 +23,186 @@ struct EnergyArgs {
   OpConst kc;            // a = 1 constants of C0
 };
 
-constexpr int kEnergyThreads = 64;
+constexpr int kEnergyLanes = 32;     // elements of a plane per block of the tensor kernel, six warps: one per load
+constexpr int kEnergyThreads = 128;  // elements of a plane per block of the energy kernel
 
-template <bool PAIRS>
-__global__ void __launch_bounds__(kEnergyThreads) k_energy(const EnergyArgs A) {
-  const int n = A.n, L = A.loads;
-  const size_t N = size_t(n) * n * n;
-  extern __shared__ double Qsm[];  // [loads][21][kEnergyThreads]
-  __shared__ double red[21 * 32];
-  const int t = threadIdx.x;
-  double acc[21];
+// Both kernels march planes of elements along z: a thread owns one column of elements of one load and keeps the
+// transform of its lower face, so a step reads one face (4 nodes). They are bound by the latency of these loads
+// and by FP64 arithmetic. Holding whole elements in shared memory for all loads, one thread per element, left
+// 192 threads on an SM and read every node 8 times. Six loads, us, that form / this one: tensor n = 32 56 / 14,
+// 54 127 / 37, 96 622 / 161; energies 54 46 / 17, 96 313 / 74.
+
+// x/y transform of the four nodes of a face of the column, per component
+struct EnergyColumn {
+  const double* u;            // the load's vector
+  unsigned o00, o10, o01, o11, plane;
+  __device__ EnergyColumn(const double* ul, int n, int x, int y) : u(ul), plane(3u * n * n) {
+    const unsigned x1 = x + 1 == n ? 0 : x + 1, y1 = y + 1 == n ? 0 : y + 1;
+    o00 = 3u * (unsigned(y) * n + x); o10 = 3u * (unsigned(y) * n + x1);
+    o01 = 3u * (y1 * n + x); o11 = 3u * (y1 * n + x1);
+  }
+  __device__ __forceinline__ void face(unsigned z, double (&F)[4][3]) const {
+    const double* p = u + z * plane;
 #pragma unroll
-  for (int k = 0; k < 21; ++k) acc[k] = 0.0;
-  const double h = 1.0 / n, invv = double(n) * n * n;
-  // each thread only touches its own column of Qsm: no block synchronisation inside the loop
-  for (size_t ee = size_t(blockIdx.x) * blockDim.x + t; ee < N; ee += size_t(gridDim.x) * blockDim.x) {
-    const int x = int(ee % n), y = int((ee / n) % n), z = int(ee / (size_t(n) * n));
-    const double ae = A.a[ee];
-    for (int l = 0; l < L; ++l) {
-      const double* m = A.macros + 6 * l;
-      // symmetric strain tensor of the engineering Voigt vector
-      const double E[3][3] = {{m[0], m[5] / 2, m[4] / 2}, {m[5] / 2, m[1], m[3] / 2}, {m[4] / 2, m[3] / 2, m[2]}};
-      double v[8][3];
-      const double* ul = A.u + size_t(l) * 3 * N;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const int bx = b & 1, by = (b >> 1) & 1, bz = (b >> 2) & 1;
-        const size_t node = (size_t(wrapi(z + bz, n)) * n + wrapi(y + by, n)) * n + wrapi(x + bx, n);
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          v[b][c] = ul[3 * node + c] + (E[c][0] * bx + E[c][1] * by + E[c][2] * bz) * h;
-      }
-      double Q[8][3];
-      hadamard8<double>(v, Q);
-#pragma unroll
-      for (int mm = 1; mm < 8; ++mm)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) Qsm[(size_t(l) * 21 + (mm - 1) * 3 + c) * kEnergyThreads + t] = Q[mm][c];
-      if (!PAIRS || A.e) {
-        double P[8][3];
-        element_modal<double>(Q, 1.0, A.kc, P);
-        double s = 0.0;
-#pragma unroll
-        for (int mm = 1; mm < 8; ++mm)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) s += Q[mm][c] * P[mm][c];
-        if (A.e) A.e[size_t(l) * N + ee] = s * invv;
-      }
-    }
-    if (PAIRS) {
-      int k = 0;
-      for (int j = 0; j < L; ++j) {
-        double Qj[8][3], Pj[8][3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) Qj[0][c] = 0.0;
-#pragma unroll
-        for (int mm = 1; mm < 8; ++mm)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) Qj[mm][c] = Qsm[(size_t(j) * 21 + (mm - 1) * 3 + c) * kEnergyThreads + t];
-        element_modal<double>(Qj, 1.0, A.kc, Pj);
-        for (int i = 0; i <= j; ++i, ++k) {
-          double s = 0.0;
-#pragma unroll
-          for (int mm = 1; mm < 8; ++mm)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) s += Qsm[(size_t(i) * 21 + (mm - 1) * 3 + c) * kEnergyThreads + t] * Pj[mm][c];
-          if (k < 21) acc[k] += ae * s;
-        }
-      }
+    for (int c = 0; c < 3; ++c) {
+      const double v00 = __ldg(p + o00 + c), v10 = __ldg(p + o10 + c);
+      const double v01 = __ldg(p + o01 + c), v11 = __ldg(p + o11 + c);
+      const double s0 = v10 + v00, d0 = v10 - v00, s1 = v11 + v01, d1 = v11 - v01;
+      F[0][c] = s1 + s0; F[1][c] = d1 + d0; F[2][c] = s1 - s0; F[3][c] = d1 - d0;
     }
   }
-  if constexpr (!PAIRS) {
-    return;
-  } else {
-  // block reduction of the 21 pair sums
+};
+
+// Modes of u + the affine field of the macro strain m on the element between the faces F0 (below) and F1, which
+// becomes the lower face of the next. The affine field is in the first-order modes only: 4 h E.
+__device__ __forceinline__ void energy_modes(const EnergyColumn& col, unsigned z, const double (&E)[6], double (&F0)[4][3],
+                                             double (&Q)[8][3]) {
+  double F1[4][3];
+  col.face(z, F1);
 #pragma unroll
-  for (int k = 0; k < 21; ++k)
+  for (int f = 0; f < 4; ++f)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      Q[f][c] = F1[f][c] + F0[f][c];
+      Q[f + 4][c] = F1[f][c] - F0[f][c];
+      F0[f][c] = F1[f][c];
+    }
+  Q[1][0] += E[0]; Q[1][1] += E[5]; Q[1][2] += E[4];
+  Q[2][0] += E[5]; Q[2][1] += E[1]; Q[2][2] += E[3];
+  Q[4][0] += E[4]; Q[4][1] += E[3]; Q[4][2] += E[2];
+}
+
+// 4 h times the symmetric tensor (xx, yy, zz, yz, xz, xy) of an engineering Voigt strain
+__device__ __forceinline__ void energy_strain(const double* m, int n, double (&E)[6]) {
+  const double h4 = 4.0 / n;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) E[k] = (k < 3 ? m[k] : m[k] / 2) * h4;
+}
+
+__device__ __forceinline__ double energy_dot(const double (&Q)[8][3], const double (&P)[8][3]) {
+  double s = 0.0;
+#pragma unroll
+  for (int m = 1; m < 8; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s += Q[m][c] * P[m][c];
+  return s;
+}
+
+// Energies of one load per blockIdx.y, z chunk per blockIdx.z.
+__global__ void __launch_bounds__(kEnergyThreads) k_energies(const EnergyArgs A) {
+  const int n = A.n, load = blockIdx.y;
+  const unsigned nn = unsigned(n) * n, i = blockIdx.x * kEnergyThreads + threadIdx.x;
+  if (i >= nn) return;
+  const size_t N = size_t(nn) * n;
+  const int z0 = blockIdx.z * A.zc, z1 = min(z0 + A.zc, n);
+  const EnergyColumn col(A.u + size_t(load) * 3 * N, n, int(i % n), int(i / n));
+  double E[6], F0[4][3];
+  energy_strain(A.macros + 6 * load, n, E);
+  const double invv = double(n) * n * n;
+  col.face(z0, F0);
+  double* e = A.e + size_t(load) * N + i;
+#pragma unroll 1
+  for (int z = z0; z < z1; ++z) {
+    double Q[8][3], P[8][3];
+    energy_modes(col, z + 1 == n ? 0 : z + 1, E, F0, Q);
+    element_modal<double>(Q, 1.0, A.kc, P);
+    e[size_t(z) * nn] = energy_dot(Q, P) * invv;
+  }
+}
+
+// Tensor (and the energies, if asked for) of six loads: warp j owns load j. It publishes its modes, double-buffered
+// over one barrier a step, and takes the pairs (j, j + k mod 6), k = 0, 1, 2, the first three warps also k = 3: each
+// of the 21 pairs once, so that the warps' work differs by one pair. Two blocks per SM: 158 registers; with three
+// the compiler has 96 and spills.
+__global__ void __launch_bounds__(6 * kEnergyLanes, 2) k_tensor(const EnergyArgs A) {
+  const int n = A.n, lane = threadIdx.x, j = threadIdx.y;
+  const unsigned nn = unsigned(n) * n, i0 = blockIdx.x * kEnergyLanes + lane, i = i0 < nn ? i0 : 0;
+  const size_t N = size_t(nn) * n;
+  const int z0 = blockIdx.y * A.zc, z1 = min(z0 + A.zc, n);
+  extern __shared__ double Qsm[];  // [parity][load][mode, component][lane]
+  constexpr int kLoad = 21 * kEnergyLanes;
+  const EnergyColumn col(A.u + size_t(j) * 3 * N, n, int(i % n), int(i / n));
+  double E[6], F0[4][3];
+  energy_strain(A.macros + 6 * j, n, E);
+  const double invv = double(n) * n * n;
+  col.face(z0, F0);
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int z = z0; z < z1; ++z) {
+    const double ae = i0 < nn ? __ldg(A.a + size_t(z) * nn + i) : 0.0;
+    double* buf = Qsm + ((z - z0) & 1) * 6 * kLoad + lane;
+    double Q[8][3], P[8][3];
+    energy_modes(col, z + 1 == n ? 0 : z + 1, E, F0, Q);
+#pragma unroll
+    for (int m = 1; m < 8; ++m)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) buf[j * kLoad + ((m - 1) * 3 + c) * kEnergyLanes] = Q[m][c];
+    element_modal<double>(Q, 1.0, A.kc, P);
+    const double own = energy_dot(Q, P);
+    acc[0] += ae * own;
+    if (A.e && i0 < nn) A.e[size_t(j) * N + size_t(z) * nn + i] = own * invv;
+    __syncthreads();  // modes published; the other parity's have been read
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+      if (k == 3 && j >= 3) continue;
+      const double* q = buf + (j + k < 6 ? j + k : j + k - 6) * kLoad;
+      double s = 0.0;
+#pragma unroll
+      for (int m = 1; m < 8; ++m)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s += q[((m - 1) * 3 + c) * kEnergyLanes] * P[m][c];
+      acc[k] += ae * s;
+    }
+  }
+  const int blk = blockIdx.x + gridDim.x * blockIdx.y, nblk = gridDim.x * gridDim.y;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k == 3 && j >= 3) continue;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], o);
-  const int warp = t >> 5, lane = t & 31;
-  if (lane == 0)
-    for (int k = 0; k < 21; ++k) red[k * 32 + warp] = acc[k];
-  __syncthreads();
-  if (t < 21) {
+    if (lane == 0) A.partials[size_t(6 * k + j) * kMaxPartials + blk] = acc[k];
+  }
+  if (!last_block(&A.scal[0].ticket[kTicketAux2], nblk)) return;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k == 3 && j >= 3) continue;
+    const double* part = A.partials + size_t(6 * k + j) * kMaxPartials;
     double s = 0.0;
-    for (int w = 0; w < kEnergyThreads / 32; ++w) s += red[t * 32 + w];
-    A.partials[size_t(t) * kMaxPartials + blockIdx.x] = s;
-  }
-  if (!last_block(&A.scal[0].ticket[kTicketAux2], gridDim.x)) return;
-  if (t < 32) {
-    for (int k = 0; k < 21; ++k) {
-      const double s = warp_sum_partials(A.partials + size_t(k) * kMaxPartials, gridDim.x);
-      if (t == 0) red[k] = s;
-    }
-    __syncwarp();
-    if (t == 0) {
-      int kk = 0;
-      for (int j = 0; j < L; ++j)
-        for (int i = 0; i <= j; ++i, ++kk) {
-          const double v = red[kk] * invv / double(N);
-          A.C[i * 6 + j] = v;
-          A.C[j * 6 + i] = v;
-        }
+    for (int b = lane; b < nblk; b += 32) s += __ldcg(part + b);
+    s = warp_reduce(s, lane, 32);
+    if (lane == 0) {
+      const int o = j + k < 6 ? j + k : j + k - 6;
+      const double v = s * invv / double(N);
+      A.C[o * 6 + j] = v;
+      A.C[j * 6 + o] = v;
     }
   }
+}
+
+// z chunks: the most even filling of the chip's `slots` blocks, counting the face that a chunk reads beyond its own;
+// at most `most` blocks.
+static int energy_chunk(int n, long columns, long slots, long most) {
+  double top = -1.0;
+  int best = n;
+  for (int nch = 1; nch <= (n + 3) / 4; ++nch) {
+    const int zc = (n + nch - 1) / nch, chunks = (n + zc - 1) / zc;
+    const long blocks = columns * chunks, waves = (blocks + slots - 1) / slots;
+    if (blocks > most) break;
+    const double eff = double(n) / (double(chunks) * (zc + 1)) * double(blocks) / double(waves * slots);
+    if (eff > top + 1e-9) { top = eff; best = zc; }
   }
+  return best;
+}
+
+static int launch_tensor(EnergyArgs& A, cudaStream_t s) {
+  const int n = A.n;
+  const unsigned columns = unsigned((n * n + kEnergyLanes - 1) / kEnergyLanes);
+  A.zc = energy_chunk(n, columns, 2 * 148, kMaxPartials);
+  const size_t smem = size_t(2) * 6 * 21 * kEnergyLanes * sizeof(double);
+  const cudaError_t e = cudaFuncSetAttribute(k_tensor, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (e != cudaSuccess) return set_cuda_error(e);
+  k_tensor<<<dim3(columns, unsigned((n + A.zc - 1) / A.zc)), dim3(kEnergyLanes, 6), smem, s>>>(A);
+  return check_launch();
 }
 
 static EnergyArgs energy_args(pgj_ctx* c, int loads, const double* u, const double* macros_dev) {
@@ -141,10 +217,9 @@ int launch_energies(pgj_ctx* c, int loads, const double* u, const double* macros
   if (loads < 1 || loads > kMaxLoads) return PGJ_ERR_ARGUMENT;
   EnergyArgs A = energy_args(c, loads, u, macros_dev);
   A.e = e;
-  const unsigned blocks = unsigned((c->N + kEnergyThreads - 1) / kEnergyThreads);
-  const size_t smem = size_t(loads) * 21 * kEnergyThreads * sizeof(double);
-  cudaFuncSetAttribute(k_energy<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  k_energy<false><<<blocks, kEnergyThreads, smem, s>>>(A);
+  const unsigned columns = unsigned((c->n * c->n + kEnergyThreads - 1) / kEnergyThreads);
+  A.zc = energy_chunk(c->n, long(columns) * loads, 4 * 148, 1L << 40);
+  k_energies<<<dim3(columns, loads, unsigned((c->n + A.zc - 1) / A.zc)), kEnergyThreads, 0, s>>>(A);
   return check_launch();
 }
 
@@ -153,14 +228,7 @@ int launch_effective_tensor(pgj_ctx* c, const double* a, const double* u, double
   A.a = a;
   A.C = C;
   A.e = e;
-  unsigned blocks = 4 * 148;
-  const unsigned need = unsigned((c->N + kEnergyThreads - 1) / kEnergyThreads);
-  if (blocks > need) blocks = need;
-  if (blocks > unsigned(kMaxPartials)) blocks = kMaxPartials;
-  const size_t smem = size_t(6) * 21 * kEnergyThreads * sizeof(double);
-  cudaFuncSetAttribute(k_energy<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  k_energy<true><<<blocks, kEnergyThreads, smem, s>>>(A);
-  return check_launch();
+  return launch_tensor(A, s);
 }
 
 }  // namespace pgj
@@ -278,13 +346,5 @@ extern "C" int pgj_effective_tensor_noalloc(int n, double lam, double mu, const 
   A.n = n; A.loads = 6; A.u = u; A.macros = voigt; A.a = a;
   A.e = nullptr; A.C = C; A.scal = scal; A.partials = partials;
   A.kc = pgj::make_opconst(n, lam, mu);
-  const size_t N = size_t(n) * n * n;
-  unsigned blocks = 4 * 148;
-  const unsigned need = unsigned((N + pgj::kEnergyThreads - 1) / pgj::kEnergyThreads);
-  if (blocks > need) blocks = need;
-  const size_t smem = size_t(6) * 21 * pgj::kEnergyThreads * sizeof(double);
-  e = cudaFuncSetAttribute(pgj::k_energy<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) return pgj::set_cuda_error(e);
-  pgj::k_energy<true><<<blocks, pgj::kEnergyThreads, smem, s>>>(A);
-  return pgj::check_launch();
+  return pgj::launch_tensor(A, s);
 }
