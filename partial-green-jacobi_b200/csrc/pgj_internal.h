@@ -165,7 +165,7 @@ int launch_green(pgj_ctx* c, int loads, int prec, const void* r, bool init, cuda
 int launch_green_pass(pgj_ctx* c, int loads, int prec, const void* r, bool init, int pass, cudaStream_t s);
 int launch_green_standalone(pgj_ctx* c, int loads, const double* r, double* z, cudaStream_t s);
 // plane transform kernels (pgj_planes.cu)
-enum PlanesMode { kPlanesUpdate = 0, kPlanesInit = 1, kPlanesSync = 2, kPlanesScale = 3 };
+enum PlanesMode { kPlanesUpdate = 0, kPlanesInit = 1, kPlanesSync = 2, kPlanesScale = 3, kPlanesApply = 4 };
 const PlaneKernels* planes_find(int n, int prec);
 int planes_prepare(const PlaneKernels* k);
 // grids on which pgj_set_fused_iteration selects between the two kernel sets: two planes of transform
@@ -176,6 +176,8 @@ int launch_planes_fwd(pgj_ctx* c, int loads, int mode, cudaStream_t s, cudaGraph
 int launch_planes_z(pgj_ctx* c, int loads, bool init, cudaStream_t s);
 int launch_planes_inv(pgj_ctx* c, int loads, bool init, cudaStream_t s, cudaGraphConditionalHandle h, bool set_cond);
 int launch_planes_shat(pgj_ctx* c, int loads, cudaStream_t s);
+// z = P s G s P r of node-major FP64 vectors (FP64 contexts); r and z may be the same
+int launch_planes_apply(pgj_ctx* c, int loads, const double* r, double* z, cudaStream_t s);
 // copies the scale fields of the loads' designs by component, in the context precision (pgj_resident.cu)
 int launch_scale_planes(pgj_ctx* c, int loads, cudaStream_t s);
 // cluster-resident PCG (pgj_resident.cu): a whole attempt's recurrence in one launch

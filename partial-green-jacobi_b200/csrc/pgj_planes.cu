@@ -122,6 +122,20 @@ int launch_planes_inv(pgj_ctx* c, int loads, bool init, cudaStream_t s, cudaGrap
   return launch(c->planes->inv, plane_grid(c, loads), c->planes->nt, c->planes->smem, A, s);
 }
 
+int launch_planes_apply(pgj_ctx* c, int loads, const double* r, double* z, cudaStream_t s) {
+  int st = launch_scale_planes(c, loads, s);
+  if (!st) st = launch_planes_shat(c, loads, s);
+  PlaneArgs A = plane_args(c, loads);
+  A.mode = kPlanesApply;
+  A.init = 1;
+  A.r64 = r;
+  A.z64 = z;
+  const PlaneKernels& k = *c->planes;
+  if (!st) st = launch(k.fwd, plane_grid(c, loads), k.nt, k.smem, A, s);
+  if (!st) st = launch(k.z, line_grid(k, loads), k.zt, k.zsmem, A, s);
+  return st ? st : launch(k.inv, plane_grid(c, loads), k.nt, k.smem, A, s);
+}
+
 // DFT(s) of the designs of `loads` loads, from the scale copy by component.
 int launch_planes_shat(pgj_ctx* c, int loads, cudaStream_t s) {
   const int designs = (loads + c->lpd - 1) / c->lpd;

@@ -27,7 +27,8 @@
 
 namespace pgj {
 
-enum PlaneMode { kPlaneUpdate = 0, kPlaneInit = 1, kPlaneSync = 2, kPlaneScale = 3 };
+// kPlaneApply: z = P s G s P r of a caller's node-major FP64 vectors, all loads, no recurrence state
+enum PlaneMode { kPlaneUpdate = 0, kPlaneInit = 1, kPlaneSync = 2, kPlaneScale = 3, kPlaneApply = 4 };
 
 struct PlaneArgs {
   int lpd, loads, cap, mode, flex, init, set_cond, forward_only;
@@ -35,7 +36,8 @@ struct PlaneArgs {
   const void* q;          // (L, 3, N) T K p
   void* r;                // (L, 3, N) T residual
   void* d;                // (L, 3, N) T correction
-  const double* r64;      // FP64 true residual, node-major (sync; FP64 init)
+  const double* r64;      // FP64 true residual, node-major (sync; FP64 init); apply: the caller's vector
+  double* z64;            // apply: the caller's result
   const void* sp;         // (designs, 3, N) T scale
   void* spec;             // (L, 3, n, n ns) complex T
   const void* shat;       // (designs, 3, n, n ns) complex T: DFT of the scale
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
     A.counters[3] += 1;  // replacements taken (launch accounting)
     cudaGraphSetConditional(A.h, 0u);
   }
-  if (mode == kPlaneSync ? S.reliable == 0 : (mode != kPlaneScale && S.active == 0)) return;
+  if (mode == kPlaneSync ? S.reliable == 0 : (mode != kPlaneScale && mode != kPlaneApply && S.active == 0)) return;
   C* buf = reinterpret_cast<C*>(smem);
   C* tw = reinterpret_cast<C*>(smem + Cfg::plane);
   double* red = reinterpret_cast<double*>(smem + Cfg::o_red);
@@ -166,7 +168,8 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
   } else {
     // transform r as it stands: from the FP64 residual (sync; first direction in FP64), held (first
     // direction in FP32), or the scale itself
-    const bool from64 = mode == kPlaneSync || (sizeof(T) == 8 && mode == kPlaneInit);
+    const bool apply = sizeof(T) == 8 && mode == kPlaneApply;
+    const bool from64 = mode == kPlaneSync || apply || (sizeof(T) == 8 && mode == kPlaneInit);
     const double* g = A.r64 + size_t(load) * N3 + 3 * (size_t(z) * NN) + c;
 #pragma unroll 2
     for (int e = tid; e < H; e += NT) {
@@ -178,8 +181,12 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
         const double* gb = ga + 3 * size_t(NN);
         a = cmk<C>(T(ga[0]), T(ga[3]));
         b = cmk<C>(T(gb[0]), T(gb[3]));
-        r2[e] = a;
-        r2[H + e] = b;
+        if (apply) {
+          acc[1] += double(a.x + a.y) + double(b.x + b.y);
+        } else {
+          r2[e] = a;
+          r2[H + e] = b;
+        }
       } else if (mode == kPlaneInit) {
         a = r2[e];
         b = r2[H + e];
@@ -212,7 +219,7 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
 
   const int nblk = 3 * (N / 2), blk = c + 3 * blockIdx.y;
   double* part = A.partials + size_t(load) * kPartialQ * kMaxPartials;
-  if (mode == kPlaneUpdate) {
+  if (mode == kPlaneUpdate || (sizeof(T) == 8 && mode == kPlaneApply)) {
     block_sum<3>(acc, red);
     if (tid == 0) {
       part[blk] = acc[0];
@@ -224,7 +231,9 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
       double v[5];
 #pragma unroll
       for (int k = 0; k < 5; ++k) v[k] = warp_sum_partials(part + k * kMaxPartials, nblk);
-      if (tid == 0) {
+      if (tid == 0 && mode == kPlaneApply) {
+        for (int cc = 0; cc < 3; ++cc) S.mean_r[cc] = v[1 + cc] / double(NV);
+      } else if (tid == 0) {
         S.rz_cross = v[4];
         // same bookkeeping as the step-by-step update (k_update_ur)
         const double res2 = v[0];
@@ -266,7 +275,7 @@ __global__ void __launch_bounds__(Cfg::ZT, Cfg::ZB) k_planes_z(const __grid_cons
   constexpr int N = Cfg::N, ZT = Cfg::ZT, NS = Cfg::NS, M = Cfg::M, CS = Cfg::CS, RA = Cfg::RA, RB = Cfg::RB;
   extern __shared__ __align__(16) unsigned char smem[];
   const int load = blockIdx.y, tid = threadIdx.x;
-  if (!A.forward_only && A.scal[load].active == 0) return;
+  if (!A.forward_only && A.mode != kPlaneApply && A.scal[load].active == 0) return;
   C* buf = reinterpret_cast<C*>(smem);  // [component][z position][column]
   C* tw = buf + 3 * N * CS;
   double* red = reinterpret_cast<double*>(smem + Cfg::o_zred);
@@ -373,13 +382,14 @@ __global__ void __launch_bounds__(Cfg::ZT, Cfg::ZB) k_planes_z(const __grid_cons
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = warp_sum_partials(part + k * kMaxPartials, nblk);
     if (tid == 0) {
-      if (A.init) {
+      if (A.mode == kPlaneApply) {
+      } else if (A.init) {
         S.beta = 0.0;
       } else {
         const double rz = S.rz;
         S.beta = (A.flex ? v[0] - S.rz_cross : v[0]) / (rz != 0.0 ? rz : 1.0);
       }
-      S.rz = v[0];
+      if (A.mode != kPlaneApply) S.rz = v[0];
       for (int k = 0; k < 3; ++k) S.mean_z[k] = v[1 + k] / double(size_t(N) * N * N);
     }
   }
@@ -407,7 +417,8 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_inv(const __grid_
     }
   }
   const LoadScalars& S = A.scal[load];
-  const bool step = S.step != 0, active = S.active != 0;
+  const bool apply = sizeof(T) == 8 && A.mode == kPlaneApply;
+  const bool step = !apply && S.step != 0, active = apply || S.active != 0;
   if (!step && !active) return;
   const size_t off = size_t(load) * N3 + size_t(c) * NV + size_t(z) * NN;
   C* d2 = reinterpret_cast<C*>(static_cast<T*>(A.d) + off);
@@ -481,6 +492,12 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_inv(const __grid_
       }
       const C w0 = buf[y * PX + x], w1 = buf[y * PX + x + 1];
       const C za = cmk<C>(sa[u].x * w0.x - m, sa[u].y * w1.x - m), zb = cmk<C>(sb[u].x * w0.y - m, sb[u].y * w1.y - m);
+      if (apply) {
+        double* o = A.z64 + size_t(load) * N3 + 3 * (size_t(z) * NN) + c + 6 * size_t(e);
+        o[0] = za.x; o[3] = za.y;
+        o[3 * size_t(NN)] = zb.x; o[3 * size_t(NN) + 3] = zb.y;
+        continue;
+      }
       p2[e] = cmk<C>(za.x + beta * pa[u].x, za.y + beta * pa[u].y);
       p2[H + e] = cmk<C>(zb.x + beta * pb[u].x, zb.y + beta * pb[u].y);
       if (zp) {
