@@ -163,7 +163,7 @@ int pgj_iteration_cap(pgj_ctx* ctx);
 /* Direction update of the FP32 recurrences of a PGJ_FP32 context (no reference counterpart; FP64
  * contexts keep the reference's beta = r.z / r_prev.z_prev): 1 selects the flexible (Polak-Ribiere)
  * form beta = r.(z - z_prev) / r_prev.z_prev, which keeps the new direction locally orthogonal when
- * the FP32 preconditioner apply is inexact (the slab-fused iteration stores z for the next
+ * the FP32 preconditioner apply is inexact (the four-kernel iteration stores z for the next
  * iteration; the step-by-step one reads it back from the last Green output). PGJ_ERR_UNSUPPORTED for
  * PGJ_FP64 contexts. Default 0. */
 int pgj_set_flexible_beta(pgj_ctx* ctx, int on);
@@ -204,9 +204,9 @@ int pgj_set_fused_iteration(pgj_ctx* ctx, int on);
  * block, out[1] operator z-planes per block, out[2] rows per x-pass block, out[3] / out[4] kx columns
  * per y / z-pass block, out[5] fused iteration flag. */
 int pgj_tile_shapes(pgj_ctx* ctx, int* out);
-/* The context's tile configuration as the tile table records it (no reference counterpart): out[0..3]
- * operator rows per block, z-planes per block, plane buffers, occupancy variant; out[4..6] requested FFT
- * rows per x block, y chunks, z chunks; out[7] fused iteration flag; out[8] where the shapes came from
+/* The context's tile configuration (no reference counterpart): out[0..3]
+ * operator rows per block, z-planes per block, 0, blocks per SM; out[4..6] requested FFT
+ * rows per x block, y chunks, z chunks; out[7] fused iteration flag; out[8] where the FFT tiles came from
  * (0 timed at creation, 1 the tile table built in, 2 environment override). */
 int pgj_tile_config(pgj_ctx* ctx, int* out);
 

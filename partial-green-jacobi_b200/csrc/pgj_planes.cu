@@ -2,11 +2,11 @@
 //
 // Measured, three kernels per iteration (forward / z / inverse), six loads, one B200, us, against the row-packed
 // slab kernels and per-line z passes that these replaced (or, where their slab did not fit, the seven
-// step-by-step kernels): FP64 n = 48 22 / 21 / 25 against 59 / 35 / 33; n = 64 67 / 29 / 69 against
+// step-by-step kernels): FP64 n = 48 21 / 21 / 14 against 59 / 35 / 33; n = 64 66 / 28 / 53 against
 // 91 / 64 / 50 (the old forward kernel carried the iterate's update, which the inverse one does now);
-// n = 80 118 / 75 / 128 against 254 / 162 / 126; n = 96 188 / 112 / 208 against 1049. FP32 n = 48
-// 19 / 17 / 16 against 40 / 31 / 27; n = 64 26 / 21 / 29 against 47 / 35 / 27; n = 96 88 / 61 / 116 against
-// 178 / 131 / 123; n = 128 212 / 176 / 254 against 1307.
+// n = 80 120 / 75 / 101 against 254 / 162 / 126; n = 96 185 / 113 / 168 against 1049. FP32 n = 48
+// 19 / 17 / 10 against 40 / 31 / 27; n = 64 25 / 21 / 19 against 47 / 35 / 27; n = 96 87 / 61 / 83 against
+// 178 / 131 / 123; n = 128 235 / 178 / 216 against 1307.
 #include "pgj_planes.cuh"
 #include <cstring>
 #include <mutex>

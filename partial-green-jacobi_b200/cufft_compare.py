@@ -9,7 +9,7 @@ symbol (1/N folded in); C2R with norm='forward'; z = s w - mean(s w). It is buil
 (cuFFT plans, elementwise kernels) in FP64 and in FP32, with the symbol from pgj_green_symbol.
 Against it: pgj_precondition (libpgj's standalone FP64 apply: five shared-memory FFT passes with the
 symbol, scalings and projection fused) and, from pgj_profile_iteration, the transform kernels of
-the slab-fused PCG iteration (which also carry the recurrence's vector updates). Prints one JSON line
+the four-kernel PCG iteration (which also carry the recurrence's vector updates). Prints one JSON line
 with CUDA-event times (ms) and the relative difference of the two FP64 results.
 """
 from __future__ import annotations

@@ -7,8 +7,8 @@ Builds a context for the seeded baseline design (n, Emin=1e-6, alpha=0.5, paper 
 certification and first direction, then times `reps` iterations kernel by kernel through
 pgj_profile_iteration (the same kernels the solve graphs launch, issued directly so that a profiler
 sees each launch). Prints the tile shapes, the iteration time and per-kernel times with the
-algorithmic bytes per second. Tile autotuners can be pinned with PGJ_STENCIL_TY / PGJ_STENCIL_ZC /
-PGJ_FFT_RB / PGJ_FFT_NKY / PGJ_FFT_NKZ.
+algorithmic bytes per second. The step-by-step FFT tiles can be pinned with PGJ_FFT_RB /
+PGJ_FFT_NKY / PGJ_FFT_NKZ.
 """
 import argparse
 import sys

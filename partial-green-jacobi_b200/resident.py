@@ -247,7 +247,7 @@ class Operator:
 
     @property
     def fused_iteration(self) -> bool:
-        """True when one PCG iteration runs as four kernels (slab-fused updates and transforms)."""
+        """True when one PCG iteration runs as four kernels (updates fused with the transforms)."""
         return bool(_lib.lib().pgj_fused_iteration(self._ctx))
 
     def set_fused_iteration(self, on: bool) -> None:
