@@ -198,7 +198,7 @@ static int capture_into(cudaGraph_t body, F&& fn) {
 
 // Mixed reliable-update iteration (FP32 recurrence, inner records active):
 // operator, update, IF(any load flagged){x += d; r64 = f - K64 x; r = T(r64)}, Green, p update.
-static int capture_iteration_rel(pgj_ctx* c, int L, cudaStream_t s, cudaGraphConditionalHandle hw) {
+static int capture_iteration_rel(pgj_ctx* c, int L, cudaStream_t s, cudaGraphConditionalHandle hw, bool last) {
   int st;
   const bool fused = c->four != 0;
   if ((st = launch_recurrence_operator(c, L, PGJ_FP32, s))) return st;
@@ -225,10 +225,10 @@ static int capture_iteration_rel(pgj_ctx* c, int L, cudaStream_t s, cudaGraphCon
   if (st) return st;
   if (fused) {
     if ((st = launch_planes_z(c, L, false, s))) return st;
-    return launch_planes_inv(c, L, false, s, hw, true);
+    return launch_planes_inv(c, L, false, s, hw, last);
   }
   if ((st = launch_green(c, L, PGJ_FP32, c->r, false, s))) return st;
-  return launch_update_p(c, L, PGJ_FP32, false, s, hw, true);
+  return launch_update_p(c, L, PGJ_FP32, false, s, hw, last);
 }
 
 static int end_capture(cudaStream_t s, cudaGraph_t* g, int st) {
@@ -237,6 +237,13 @@ static int end_capture(cudaStream_t s, cudaGraph_t* g, int st) {
   if (e != cudaSuccess) return set_cuda_error(e);
   return PGJ_OK;
 }
+
+// Iterations in one pass of the loop. Looking at the condition between passes costs 4 to 6 us, as much as a kernel
+// of a small grid. Loads that have stopped skip the rest of a pass: at most three idle iterations of about 10 us
+// end an attempt. Per iteration with one / two / four in a pass, us: FP64 n = 48 86.6 / 83.6 / 82.2, 64 186.5 /
+// 183.4 / 181.8; mixed n = 48 70.5 / 67.8 / 66.2, 64 110.2 / 107.5 / 105.4, 96 327.5 / 325.8 / 326.2. The eight
+// kernels of the step-by-step form run large grids, where it makes no difference.
+static int iterations_per_body(const pgj_ctx* c) { return c->four ? 4 : 1; }
 
 // Appends to the capture on `s`: directions init, then WHILE(any load active){iteration}.
 static int capture_pcg(pgj_ctx* c, int L, cudaStream_t s, bool reliable = false) {
@@ -247,7 +254,10 @@ static int capture_pcg(pgj_ctx* c, int L, cudaStream_t s, bool reliable = false)
   if (!st) st = add_conditional(s, &h, 1, cudaGraphCondTypeWhile, &body);
   if (st) return st;
   return capture_into(body, [&](cudaStream_t s2) {
-    return reliable ? capture_iteration_rel(c, L, s2, h) : capture_iteration(c, L, s2, h, true);
+    int r = 0;
+    for (int left = iterations_per_body(c); left > 0 && !r; --left)
+      r = reliable ? capture_iteration_rel(c, L, s2, h, left == 1) : capture_iteration(c, L, s2, h, left == 1);
+    return r;
   });
 }
 
@@ -661,7 +671,7 @@ int pgj_solve_wait(pgj_ctx* c, pgj_load_info* info, void* stream) {
   // loop body: operator, update, 5 Green passes, p update (fused: operator and three plane kernels), plus the
   // IF-condition kernel of the step-by-step reliable-update form; the first direction is 6 kernels after the mask /
   // recurrence-start kernel, and the plane kernels' FP64 form ends with x += d
-  const long long body = c->four ? 4 : 8 + (c->prec == PGJ_FP32 ? 1 : 0);
+  const long long body = iterations_per_body(c) * (c->four ? 4 : 8 + (c->prec == PGJ_FP32 ? 1 : 0));
   const long long first = first_direction_launches(c);
   if (uses_resident(c))  // scale copy, the resident recurrence, certify, decide
     c->last_launches = 2 + 3 + attempts * (2 + 3 + 1);
@@ -730,7 +740,7 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
       ++sweeps;
       if ((e = read_state(true)) != cudaSuccess) return set_cuda_error(e);
       // sweep: inner start + first direction, loop bodies, x += d, 3 certification kernels
-      launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * body[0] + 1 + 3;
+      launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * iterations_per_body(c) * body[0] + 1 + 3;
       if (body[1]) { capped_by_bound = true; break; }
     }
   } else {
@@ -738,9 +748,9 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
       if ((e = cudaGraphLaunch(c->graphs->attempt, s)) != cudaSuccess) return set_cuda_error(e);
       if ((e = read_state(true)) != cudaSuccess) return set_cuda_error(e);
       if (c->prec == PGJ_FP32)  // rel start + first direction, bodies, 3 per replacement, fold + certify
-        launches += 1 + first_direction_launches(c) + (c->four ? 5LL : 9LL) * body[0] + 3LL * body[3] + 1 + 3;
+        launches += 1 + first_direction_launches(c) + (c->four ? 5LL : 9LL) * iterations_per_body(c) * body[0] + 3LL * body[3] + 1 + 3;
       else  // attempt: init mask + first direction, loop bodies, 3 certification kernels
-        launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * body[0] + 3;
+        launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * iterations_per_body(c) * body[0] + 3;
       if (body[1]) { capped_by_bound = true; break; }
       bool all, anybad, capped;
       evaluate(all, anybad, capped);
