@@ -2,9 +2,9 @@
 //
 // Measured, three kernels per iteration (forward / z / inverse), six loads, one B200, us, against the row-packed
 // slab kernels and per-line z passes that these replaced (or, where their slab did not fit, the seven
-// step-by-step kernels): FP64 n = 48 21 / 21 / 14 against 59 / 35 / 33; n = 64 66 / 28 / 53 against
+// step-by-step kernels): FP64 n = 48 21 / 21 / 14 against 59 / 35 / 33; n = 64 52 / 28 / 41 against
 // 91 / 64 / 50 (the old forward kernel carried the iterate's update, which the inverse one does now);
-// n = 80 120 / 75 / 101 against 254 / 162 / 126; n = 96 185 / 113 / 168 against 1049. FP32 n = 48
+// n = 80 108 / 75 / 99 against 254 / 162 / 126; n = 96 185 / 113 / 168 against 1049. FP32 n = 48
 // 19 / 17 / 10 against 40 / 31 / 27; n = 64 25 / 21 / 19 against 47 / 35 / 27; n = 96 87 / 61 / 83 against
 // 178 / 131 / 123; n = 128 235 / 178 / 216 against 1307.
 #include "pgj_planes.cuh"

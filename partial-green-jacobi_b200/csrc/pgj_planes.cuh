@@ -59,11 +59,16 @@ template <int N_, typename T_> struct PlaneCfg {
   static constexpr size_t plane = size_t(N) * PX * 2 * sizeof(T);
   static constexpr size_t o_red = (plane + N * 2 * sizeof(T) + 15) / 16 * 16;
   static constexpr size_t smem = o_red + 4 * 32 * 8;
-  // blocks per SM that the planes leave room for, and threads for each (a butterfly holds up to 16
-  // complex values: 64 registers in FP32, 85 in FP64 unless one block has the SM to itself)
+  // Blocks per SM: as many as keep their planes within 140 KB, at least two if they fit at all. The rest of an SM's
+  // 256 KB is the L1 that the vectors pass through: with three FP64 blocks at n = 64 (200 KB of planes) the forward
+  // and inverse kernels took 66 and 51 us, with two 52 and 41; n = 60 50 and 42 / 43 and 35; FP32 n = 90 86 and 86 /
+  // 76 and 66. Below, the third block pays: n = 48 21 and 14 against 27 and 17 with two. Threads: a butterfly holds up
+  // to 16 complex values, 64 registers in FP32, 85 in FP64; from 64 lines on 512 threads take a pass in one or two
+  // rounds (FP64 n = 80 109 against 119 us with 384), below 384 have more registers (n = 60 78 against 81 us, both).
   static constexpr int fit = int((227 * 1024) / (smem + 1024));
-  static constexpr int MINB = sizeof(T) == 4 ? (fit >= 4 ? 4 : fit) : (fit >= 3 ? 3 : fit);
-  static constexpr int NT = N <= 24 ? 128 : MINB >= 3 ? 256 : MINB == 2 ? (sizeof(T) == 4 ? 512 : 384) : 512;
+  static constexpr int most = sizeof(T) == 4 ? 4 : 3, room = int((140 * 1024) / smem);
+  static constexpr int MINB = room >= most ? most : room >= 3 ? 3 : fit >= 2 ? 2 : 1;
+  static constexpr int NT = N <= 24 ? 128 : MINB >= 3 ? 256 : sizeof(T) == 8 && MINB == 2 && N < 64 ? 384 : 512;
   static_assert(fit >= 1, "a plane pair fits");
   // z kernel
   static constexpr int CS = sizeof(T) == 4 ? 32 : 16;
