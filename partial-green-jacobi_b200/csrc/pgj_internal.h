@@ -65,6 +65,38 @@ constexpr int kAuxVoigt = 32;
 constexpr int kAuxPartials = 128;
 constexpr int kAuxDoubles = kAuxPartials + kMaxPartials;
 
+// Component means of one load's node-major vector by the blocks of a grid row (256 threads each), to dst[3].
+__device__ __forceinline__ void grid_mean3(size_t N, const double* __restrict__ u, double* dst, LoadScalars& S, double* part) {
+  double acc[3] = {0.0, 0.0, 0.0};
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x) {
+    acc[0] += u[3 * i]; acc[1] += u[3 * i + 1]; acc[2] += u[3 * i + 2];
+  }
+  __shared__ double red[96];
+  block_sum<3>(acc, red);
+  if (threadIdx.x == 0)
+    for (int k = 0; k < 3; ++k) part[k * kMaxPartials + blockIdx.x] = acc[k];
+  if (!last_block(&S.ticket[kTicketAux], gridDim.x)) return;
+  if (threadIdx.x < 32) {
+    double v[3];
+    for (int k = 0; k < 3; ++k) v[k] = warp_sum_partials(part + k * kMaxPartials, gridDim.x);
+    if (threadIdx.x == 0)
+      for (int k = 0; k < 3; ++k) dst[k] = v[k] / double(N);
+  }
+}
+
+// One design's scale field by component, by the blocks of a grid row: out[c][node] = T(s[3 node + c]).
+template <typename T>
+__device__ __forceinline__ void scale_planes_row(size_t N, int design, const double* __restrict__ s, T* __restrict__ out) {
+  s += size_t(design) * 3 * N;
+  out += size_t(design) * 3 * N;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x) {
+    const double a = s[3 * i], b = s[3 * i + 1], c = s[3 * i + 2];
+    out[i] = T(a);
+    out[N + i] = T(b);
+    out[2 * N + i] = T(c);
+  }
+}
+
 struct Layout {
   size_t a, scale, scale32, symbol, symbol32, tw, solutions, f, x, r, p, q, sw, spec, shat, partials, scal, macros,
       cond, r64, d, aux, scale_pl, halo, total;

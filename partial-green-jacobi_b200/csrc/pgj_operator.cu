@@ -137,26 +137,8 @@ __global__ void k_mean3(int n, const double* __restrict__ u, int which, LoadScal
   const size_t N = size_t(n) * n * n;
   const int load = blockIdx.y;
   if (which == 0 && scal[load].frozen) return;  // certification of a design that took its last attempt
-  const double* ul = u + size_t(load) * 3 * N;
-  double acc[3] = {0.0, 0.0, 0.0};
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x) {
-    acc[0] += ul[3 * i]; acc[1] += ul[3 * i + 1]; acc[2] += ul[3 * i + 2];
-  }
-  __shared__ double red[96];
-  block_sum<3>(acc, red);
-  double* part = partials + size_t(load) * kPartialQ * kMaxPartials;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) part[k * kMaxPartials + blockIdx.x] = acc[k];
   LoadScalars& S = scal[load];
-  if (!last_block(&S.ticket[kTicketAux], gridDim.x)) return;
-  if (threadIdx.x < 32) {
-    double v[3];
-    for (int k = 0; k < 3; ++k) v[k] = warp_sum_partials(part + k * kMaxPartials, gridDim.x);
-    if (threadIdx.x == 0) {
-      double* dst = which ? S.mean_r : S.mean_u;
-      for (int k = 0; k < 3; ++k) dst[k] = v[k] / double(N);
-    }
-  }
+  grid_mean3(N, u + size_t(load) * 3 * N, which ? S.mean_r : S.mean_u, S, partials + size_t(load) * kPartialQ * kMaxPartials);
 }
 
 __global__ void k_sub_mean3(int n, double* __restrict__ u, const LoadScalars* scal) {

@@ -122,8 +122,25 @@ int launch_planes_inv(pgj_ctx* c, int loads, bool init, cudaStream_t s, cudaGrap
   return launch(c->planes->inv, plane_grid(c, loads), c->planes->nt, c->planes->smem, A, s);
 }
 
+// What the apply needs beforehand, in one launch: rows y < designs of the grid copy the designs' scale fields by
+// component, the others form the means of the loads' vectors (n = 64, six loads: 139.4 us without the means, 141.1
+// with them).
+static __global__ void __launch_bounds__(256) k_apply_prepare(size_t N, int designs, const double* __restrict__ scale,
+                                                              double* __restrict__ sp, const double* __restrict__ r,
+                                                              LoadScalars* scal, double* partials) {
+  if (int(blockIdx.y) < designs) {
+    scale_planes_row(N, blockIdx.y, scale, sp);
+    return;
+  }
+  const int load = int(blockIdx.y) - designs;
+  grid_mean3(N, r + size_t(load) * 3 * N, scal[load].mean_r, scal[load], partials + size_t(load) * kPartialQ * kMaxPartials);
+}
+
 int launch_planes_apply(pgj_ctx* c, int loads, const double* r, double* z, cudaStream_t s) {
-  int st = launch_scale_planes(c, loads, s);
+  const int designs = (loads + c->lpd - 1) / c->lpd;
+  k_apply_prepare<<<dim3(148, unsigned(designs + loads)), 256, 0, s>>>(size_t(c->N), designs, c->scale, c->scale_pl, r,
+                                                                       c->scal, c->partials);
+  int st = check_launch();
   if (!st) st = launch_planes_shat(c, loads, s);
   PlaneArgs A = plane_args(c, loads);
   A.mode = kPlanesApply;

@@ -27,7 +27,9 @@
 
 namespace pgj {
 
-// kPlaneApply: z = P s G s P r of a caller's node-major FP64 vectors, all loads, no recurrence state
+// kPlaneApply: z = P s G s P r of a caller's node-major FP64 vectors, all loads, no recurrence state. The mean of r
+// comes from a pass of its own and leaves before the transforms: a recurrence's residual has next to none, a caller's
+// vector may have one of any size, and taking that out in Fourier space would leave its rounding in z.
 enum PlaneMode { kPlaneUpdate = 0, kPlaneInit = 1, kPlaneSync = 2, kPlaneScale = 3, kPlaneApply = 4 };
 
 struct PlaneArgs {
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
     const bool apply = sizeof(T) == 8 && mode == kPlaneApply;
     const bool from64 = mode == kPlaneSync || apply || (sizeof(T) == 8 && mode == kPlaneInit);
     const double* g = A.r64 + size_t(load) * N3 + 3 * (size_t(z) * NN) + c;
+    const T m = apply ? T(S.mean_r[c]) : T(0);
 #pragma unroll 2
     for (int e = tid; e < H; e += NT) {
       const int y = e / (N / 2), x = 2 * (e - y * (N / 2));
@@ -187,7 +190,8 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
         a = cmk<C>(T(ga[0]), T(ga[3]));
         b = cmk<C>(T(gb[0]), T(gb[3]));
         if (apply) {
-          acc[1] += double(a.x + a.y) + double(b.x + b.y);
+          a = cmk<C>(a.x - m, a.y - m);
+          b = cmk<C>(b.x - m, b.y - m);
         } else {
           r2[e] = a;
           r2[H + e] = b;
@@ -220,11 +224,11 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
     sp[k] = cmk<C>(T(0.5) * (zk.x + zn.x), T(0.5) * (zk.y - zn.y));
     sp[M + k] = cmk<C>(T(0.5) * (zk.y + zn.y), T(0.5) * (zn.x - zk.x));
   }
-  if (mode == kPlaneInit || mode == kPlaneScale) return;
+  if (mode == kPlaneInit || mode == kPlaneScale || mode == kPlaneApply) return;
 
   const int nblk = 3 * (N / 2), blk = c + 3 * blockIdx.y;
   double* part = A.partials + size_t(load) * kPartialQ * kMaxPartials;
-  if (mode == kPlaneUpdate || (sizeof(T) == 8 && mode == kPlaneApply)) {
+  if (mode == kPlaneUpdate) {
     block_sum<3>(acc, red);
     if (tid == 0) {
       part[blk] = acc[0];
@@ -236,9 +240,7 @@ __global__ void __launch_bounds__(Cfg::NT, Cfg::MINB) k_planes_fwd(const __grid_
       double v[5];
 #pragma unroll
       for (int k = 0; k < 5; ++k) v[k] = warp_sum_partials(part + k * kMaxPartials, nblk);
-      if (tid == 0 && mode == kPlaneApply) {
-        for (int cc = 0; cc < 3; ++cc) S.mean_r[cc] = v[1 + cc] / double(NV);
-      } else if (tid == 0) {
+      if (tid == 0) {
         S.rz_cross = v[4];
         // same bookkeeping as the step-by-step update (k_update_ur)
         const double res2 = v[0];
@@ -326,7 +328,10 @@ __global__ void __launch_bounds__(Cfg::ZT, Cfg::ZB) k_planes_z(const __grid_cons
     }
     const int kx = (m0 + ml) % NS;
     const double wgt = (kx == 0 || kx == N / 2) ? 1.0 : 2.0;
-    const T mx = T(A.scal[load].mean_r[0]), my = T(A.scal[load].mean_r[1]), mz = T(A.scal[load].mean_r[2]);
+    // DFT(s.(r - mean r)) = DFT(s.r) - mean r . DFT(s); apply: the mean is already out
+    const bool out = A.mode == kPlaneApply;
+    const T mx = out ? T(0) : T(A.scal[load].mean_r[0]), my = out ? T(0) : T(A.scal[load].mean_r[1]);
+    const T mz = out ? T(0) : T(A.scal[load].mean_r[2]);
     double part[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int k = 0; k < RB; ++k) {
@@ -335,7 +340,6 @@ __global__ void __launch_bounds__(Cfg::ZT, Cfg::ZB) k_planes_z(const __grid_cons
       const T c0 = __ldg(sym + kk), c1 = __ldg(sym + Nh + kk), c2 = __ldg(sym + 2 * Nh + kk);
       const T c3 = __ldg(sym + 3 * Nh + kk), c4 = __ldg(sym + 4 * Nh + kk), c5 = __ldg(sym + 5 * Nh + kk);
       const C s0 = __ldg(sh + kk), s1 = __ldg(sh + Nh + kk), s2 = __ldg(sh + 2 * Nh + kk);
-      // DFT(s.(r - mean r)) = DFT(s.r) - mean r . DFT(s)
       const C x = cmk<C>(v[0][k].x - mx * s0.x, v[0][k].y - mx * s0.y);
       const C y = cmk<C>(v[1][k].x - my * s1.x, v[1][k].y - my * s1.y);
       const C z = cmk<C>(v[2][k].x - mz * s2.x, v[2][k].y - mz * s2.y);

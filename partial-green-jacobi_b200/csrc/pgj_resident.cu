@@ -88,17 +88,9 @@ const ResidentKernel* resident_prepare(int n, int prec) {
   return it->second ? k : nullptr;
 }
 
-// out[c][node] = T(s[3 node + c]) for every design
 template <typename T>
 __global__ void k_scale_planes(size_t N, const double* __restrict__ s, T* __restrict__ out) {
-  s += size_t(blockIdx.y) * 3 * N;
-  out += size_t(blockIdx.y) * 3 * N;
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += size_t(gridDim.x) * blockDim.x) {
-    const double a = s[3 * i], b = s[3 * i + 1], c = s[3 * i + 2];
-    out[i] = T(a);
-    out[N + i] = T(b);
-    out[2 * N + i] = T(c);
-  }
+  scale_planes_row(N, blockIdx.y, s, out);
 }
 
 int launch_scale_planes(pgj_ctx* c, int loads, cudaStream_t s) {
