@@ -90,7 +90,8 @@ struct ConeSmem {
 };
 
 // Radius of the tap table (max |offset|) if it fits the tile form, else -1; the tile form's tap table is
-// then staged in `sm`. Called by every thread of a 32 x 8 block.
+// then staged in `sm`. Called by every thread of a 32 x 8 block. A weight that is not finite does not fit: a tap
+// that falls outside the grid would not add zero.
 __device__ __forceinline__ int cone_stage(ConeSmem& sm, const int32_t* __restrict__ offsets,
                                           const double* __restrict__ weights, int count) {
   const int tid = flat_tid();
@@ -103,6 +104,8 @@ __device__ __forceinline__ int cone_stage(ConeSmem& sm, const int32_t* __restric
     const int d = offsets[j];
     r = max(r, d < -kConeR || d > kConeR ? kConeR + 1 : abs(d));
   }
+  for (int j = tid; j < count; j += kConeX * kConeY)
+    if (!isfinite(weights[j])) r = kConeR + 1;
   atomicMax(&radius, r);
   __syncthreads();
   r = radius;
