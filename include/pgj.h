@@ -210,10 +210,11 @@ int pgj_tile_shapes(pgj_ctx* ctx, int* out);
  * (0 timed at creation, 1 the tile table built in, 2 environment override). */
 int pgj_tile_config(pgj_ctx* ctx, int* out);
 
-/* Failure-detection self-test (no reference counterpart): runs the bounded device wait used by the
- * kernels' TMA staging on an mbarrier that nothing completes, giving up after `tries` polls.
- * Returns PGJ_ERR_TIMEOUT when the wait expired and was reported (the expected outcome); the
- * context stays usable. Never faults or hangs: no copy is issued and the wait is bounded. */
+/* Failure-detection self-test (no reference counterpart): runs the bounded device waits of the resident
+ * solver (an mbarrier that nothing arrives at) and of the design updates (a grid barrier one arrival
+ * short), giving up after about `tries` microseconds each. Returns PGJ_ERR_TIMEOUT when both expired and
+ * were reported, the design update's also in the record of an enqueue-only call (the expected
+ * outcome); the context stays usable. Never faults or hangs: the waits are bounded. */
 int pgj_selftest_wait_timeout(pgj_ctx* ctx, int tries, void* stream);
 
 /* ------------------------------------------------------------------ responses
@@ -249,13 +250,17 @@ int pgj_paper_project(int n, const double* t, const double* hs, double beta, dou
  * host `steps` (bisections taken) and `change` (max |xnew - x|), read back with one stream
  * synchronisation. With steps and change both NULL the update is only enqueued (no
  * synchronisation); the bisections taken and the change are then left at scratch[4 n^3 + 3] and
- * scratch[4 n^3 + 4]. scratch: 4 n^3 + 512 float64 device. */
+ * scratch[4 n^3 + 4]. An update whose blocks waited in vain for each other (20 s; other work held the
+ * SMs they needed) ends with xnew unfinished: the call that synchronises returns PGJ_ERR_TIMEOUT, an
+ * enqueue-only one leaves -1 steps and a NaN change. scratch: 4 n^3 + 512 float64 device. */
 int pgj_paper_oc(int n, const int32_t* offsets, const double* weights, int count, const double* x,
                  const double* ph, const double* dp, const double* hs, const double* energy,
                  double volume, double beta, double eta, double emin, double move, double exponent,
                  double floor_, double* xnew, double* scratch, int* steps, double* change, void* stream);
 /* Study I chain: periodic separable Gaussian (sigma = 0.9 n/32), tanh projection at 1/2, SIMP
- * eta=1e-4 and 45-step OC (ResidentOuter, exp/asg_gpu_resident_20261103/outer.py:12-59, outer.cu:7-37). */
+ * eta=1e-4 and 45-step OC (ResidentOuter, exp/asg_gpu_resident_20261103/outer.py:12-59, outer.cu:7-37).
+ * pgj_study1_oc with change NULL only enqueues; steps, change and the mark of a wait that expired are left in
+ * scratch as by pgj_paper_oc. */
 int pgj_gaussian_filter(int n, const double* weights, int radius, const double* x, double* y,
                         double* scratch, void* stream);
 int pgj_study1_project(int n, const double* t, double beta, double* ph, double* dp, double* a, void* stream);

@@ -39,23 +39,6 @@ __device__ __forceinline__ void tma_row(void* dst, const void* src, unsigned byt
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait: gives up after kMaxTries polls (each poll may suspend briefly in hardware).
-constexpr int kMaxTries = 1 << 20;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, int max_tries = kMaxTries) {
-  for (int i = 0; i < max_tries; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
-}
-
 // Bulk store shared -> global (the async proxy reads shared memory; make generic writes visible first
 // with fence_proxy_async() and a block barrier, and wait for the reads before the buffer is reused
 // or the block exits).

@@ -818,13 +818,15 @@ int pgj_selftest_wait_timeout(pgj_ctx* c, int tries, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(c->cond + 6, 0, sizeof(int), s);
   if (e != cudaSuccess) return set_cuda_error(e);
-  int st = launch_wait_selftest(tries, c->cond + 6, s);
+  int st = launch_cluster_wait_selftest(tries, c->cond + 6, s);
+  bool expired = false;
+  if (!st) st = grid_wait_selftest(tries, c->partials, &expired, s);
   if (st) return st;
   int flag = 0;
   e = cudaMemcpyAsync(&flag, c->cond + 6, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return set_cuda_error(e);
-  return flag ? PGJ_ERR_TIMEOUT : PGJ_OK;
+  return flag && expired ? PGJ_ERR_TIMEOUT : PGJ_OK;
 }
 
 int pgj_profile_iteration(pgj_ctx* c, int loads, const double* macros, int reps, double* ms, double* bytes,

@@ -254,7 +254,9 @@ struct DesignScope {
 int set_cuda_error(cudaError_t e);
 // one-time kernel attributes (dynamic shared memory limits); called at context creation
 int prepare_rows();
-int launch_wait_selftest(int tries, int* flag, cudaStream_t s);
+// the bounded waits of the OC updates (pgj_outer.cu) and the resident kernel, with nothing to complete them
+int grid_wait_selftest(int limit_us, double* record, bool* expired, cudaStream_t s);
+int launch_cluster_wait_selftest(int limit_us, int* flag, cudaStream_t s);
 // times candidate tile shapes of the Green passes and keeps the fastest
 int autotune_fft(pgj_ctx* c, cudaStream_t s);
 int prepare_fft_kernels();

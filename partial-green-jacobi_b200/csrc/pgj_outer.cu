@@ -35,7 +35,7 @@ struct GridBar {
 };
 constexpr unsigned long long kGridWaitNs = 20000000000ull;
 
-__device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned& target) {
+__device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned& target, unsigned long long limit = kGridWaitNs) {
   target += gridDim.x;
   __syncthreads();
   int dead = 0;
@@ -50,7 +50,7 @@ __device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned& target) {
         dead = *(volatile int*)&b->dead;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
         if (t0 == 0) t0 = t;
-        if (dead || t - t0 > kGridWaitNs) {
+        if (dead || t - t0 > limit) {
           dead = 1;
           *(volatile int*)&b->dead = 1;
           break;
@@ -59,6 +59,20 @@ __device__ __forceinline__ bool grid_barrier(GridBar* b, unsigned& target) {
     }
   }
   return __syncthreads_or(dead) == 0;
+}
+
+// Leaves the mark of an update that gave up in the record a caller without a synchronisation reads: -1 steps and a
+// NaN change. grid_max takes the largest bit pattern, which keeps the NaN whatever other blocks still add.
+__device__ __forceinline__ void oc_gave_up(double* bounds) {
+  if (flat_tid() != 0) return;
+  *(volatile double*)(bounds + 3) = -1.0;
+  atomicMax(reinterpret_cast<unsigned long long*>(bounds + 4), 0x7ff8000000000000ull);
+}
+
+// Self-test: a barrier that needs one more arrival than there are blocks.
+__global__ void k_grid_wait_selftest(GridBar* bar, double* bounds, unsigned long long limit) {
+  unsigned target = 1;
+  if (!grid_barrier(bar, target, limit)) oc_gave_up(bounds);
 }
 
 // --------------------------------------------------------------------------- cone filter
@@ -295,7 +309,7 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
     A.f2[i] = dp * (3 * (1 - A.emin) * (ph * ph)) * A.energy[i] / hs;
     A.f3[i] = dp / hs;
   }
-  if (!grid_barrier(A.bar, target)) return;
+  if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
   const double dN = double(N);
   for (int t = blockIdx.x; t < A.tiles; t += gridDim.x) {
     double g[kConeZ];
@@ -309,7 +323,7 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
                 A.f1[i] = v;
               });
   }
-  if (!grid_barrier(A.bar, target)) return;
+  if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
   const double te = tanh(A.beta * A.eta), den = te + tanh(A.beta * (1 - A.eta));
   double lo = 0.0, hi = 1e9, steps = 0.0;
   bool go = true;
@@ -320,7 +334,7 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
       const double v = xi * pow(fmax(1e-10, __ldcg(A.f0 + i) / mid), A.exponent);
       A.xnew[i] = fmax(A.floor_, fmax(xi - A.move, fmin(1.0, fmin(xi + A.move, v))));
     }
-    if (!grid_barrier(A.bar, target)) return;
+    if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
     double acc[1] = {0.0};
     for (int t = blockIdx.x; t < A.tiles; t += gridDim.x)
       cone_tile(sm, radius, n, A.offsets, A.weights, A.count, t, [&](size_t i) { return __ldcg(A.xnew + i); },
@@ -331,7 +345,7 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
                 });
     block_sum<1>(acc, red);
     if (tid == 0) A.partials[blockIdx.x] = acc[0];
-    if (!grid_barrier(A.bar, target)) return;
+    if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
     const double vol = sum_partials(A.partials) / dN;
     if (vol > A.volume) lo = mid; else hi = mid;
     steps += 1.0;
@@ -340,7 +354,7 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
   double m = 0.0;
   for (size_t i = first; i < N; i += stride) m = fmax(m, fabs(__ldcg(A.xnew + i) - A.x[i]));
   grid_max(m, A.bounds + 4);
-  if (blockIdx.x == 0 && tid == 0) {
+  if (blockIdx.x == 0 && tid == 0 && !*(volatile int*)&A.bar->dead) {
     A.bounds[0] = lo;
     A.bounds[1] = hi;
     A.bounds[2] = go ? 1.0 : 0.0;
@@ -554,7 +568,7 @@ __global__ void __launch_bounds__(kS1Threads) k_s1_oc(const OCArgs A) {
                [](size_t, double v) { return v; }, A.f2);
     s1_columns(buf, w, radius, n, t, [&](size_t i) { return A.dp[i]; }, [](size_t, double v) { return v; }, A.f3);
   }
-  if (!grid_barrier(A.bar, target)) return;
+  if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
   // ratio = max(g, 1e-30) / max(dv, 1e-30); the upper bound is 1e4 times its maximum
   double m = 0.0;
   for (int t = blockIdx.x; t < tasks; t += gridDim.x) {
@@ -566,7 +580,7 @@ __global__ void __launch_bounds__(kS1Threads) k_s1_oc(const OCArgs A) {
     });
   }
   grid_max(m, A.bounds + 6);
-  if (!grid_barrier(A.bar, target)) return;
+  if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
   double lo = 0.0, hi = __ldcg(A.bounds + 6) * 1e4;
   for (int it = 0; it < 45; ++it) {
     const double mid = (lo + hi) * 0.5, lam = fmax(mid, 1e-30);
@@ -581,7 +595,7 @@ __global__ void __launch_bounds__(kS1Threads) k_s1_oc(const OCArgs A) {
                    return v;
                  },
                  A.f2);
-    if (!grid_barrier(A.bar, target)) return;
+    if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
     double acc[1] = {0.0};
     for (int t = blockIdx.x; t < tasks; t += gridDim.x)
       s1_rows(buf, w, radius, n, t, A.f2, [&](size_t, double v) {
@@ -591,14 +605,14 @@ __global__ void __launch_bounds__(kS1Threads) k_s1_oc(const OCArgs A) {
       });
     block_sum<1>(acc, red);
     if (tid == 0) A.partials[blockIdx.x] = acc[0];
-    if (!grid_barrier(A.bar, target)) return;
+    if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
     if (sum_partials(A.partials) / double(N) > A.volume) lo = mid; else hi = mid;
   }
   m = 0.0;
   for (size_t i = size_t(blockIdx.x) * kS1Threads + tid; i < N; i += size_t(gridDim.x) * kS1Threads)
     m = fmax(m, fabs(__ldcg(A.xnew + i) - A.x[i]));
   grid_max(m, A.bounds + 4);
-  if (blockIdx.x == 0 && tid == 0) {
+  if (blockIdx.x == 0 && tid == 0 && !*(volatile int*)&A.bar->dead) {
     A.bounds[0] = lo;
     A.bounds[1] = hi;
     A.bounds[2] = 1.0;
@@ -681,12 +695,30 @@ int read_record(const OCScratch& w, int* steps, double* change, cudaStream_t s) 
   if (e != cudaSuccess) return set_cuda_error(e);
   GridBar bar;
   std::memcpy(&bar, host + 8, sizeof(bar));
-  if (bar.dead) return PGJ_ERR_TIMEOUT;
   if (steps) *steps = int(host[3]);
   if (change) *change = host[4];
-  return PGJ_OK;
+  return bar.dead ? PGJ_ERR_TIMEOUT : PGJ_OK;
 }
 }  // namespace
+
+namespace pgj {
+// `record`: 16 device doubles; *expired: the barrier gave up and left its mark
+int grid_wait_selftest(int limit_us, double* record, bool* expired, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(record, 0, 16 * sizeof(double), s);
+  if (e != cudaSuccess) return set_cuda_error(e);
+  const unsigned long long limit = std::min(1000ull * static_cast<unsigned long long>(limit_us), kGridWaitNs);
+  k_grid_wait_selftest<<<1, 32, 0, s>>>(reinterpret_cast<GridBar*>(record + 8), record, limit);
+  int st = check_launch();
+  if (st) return st;
+  OCScratch w = {};
+  w.bounds = record;
+  int steps = 0;
+  double change = 0.0;
+  st = read_record(w, &steps, &change, s);
+  *expired = st == PGJ_ERR_TIMEOUT && steps == -1 && std::isnan(change);
+  return st == PGJ_ERR_TIMEOUT ? PGJ_OK : st;
+}
+}  // namespace pgj
 
 extern "C" {
 

@@ -93,6 +93,26 @@ __global__ void k_scale_planes(size_t N, const double* __restrict__ s, T* __rest
   scale_planes_row(N, blockIdx.y, s, out);
 }
 
+// Self-test: an mbarrier that nothing arrives at.
+__global__ void k_cluster_wait_selftest(long long limit, int* flag) {
+  __shared__ ClusterBar bar;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar.tx[0], 1);
+    fence_mbar_init();
+    bar.dead = 0;
+  }
+  __syncthreads();
+  cluster_wait_on(&bar, &bar.tx[0], 0u, limit);
+  __syncthreads();
+  if (threadIdx.x == 0) *flag = bar.dead;
+}
+
+int launch_cluster_wait_selftest(int limit_us, int* flag, cudaStream_t s) {
+  const long long limit = 1000ll * limit_us;
+  k_cluster_wait_selftest<<<1, 32, 0, s>>>(limit < kClusterWaitClocks ? limit : kClusterWaitClocks, flag);
+  return check_launch();
+}
+
 int launch_scale_planes(pgj_ctx* c, int loads, cudaStream_t s) {
   const size_t N = size_t(c->N);
   const dim3 grid(unsigned((N + 255) / 256 < 148 ? (N + 255) / 256 : 148), unsigned((loads + c->lpd - 1) / c->lpd));

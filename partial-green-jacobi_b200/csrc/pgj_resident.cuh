@@ -160,7 +160,8 @@ __device__ __forceinline__ void cluster_arrive(ClusterBar* b, unsigned phase) { 
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(remote) : "memory");
   }
 }
-__device__ __forceinline__ void cluster_wait_on(ClusterBar* b, uint64_t* which, unsigned parity) {
+__device__ __forceinline__ void cluster_wait_on(ClusterBar* b, uint64_t* which, unsigned parity,
+                                                long long limit = kClusterWaitClocks) {
   volatile int* dead = &b->dead;
   const uint32_t at = smem_u32(which);
   const long long t0 = clock64();
@@ -173,7 +174,7 @@ __device__ __forceinline__ void cluster_wait_on(ClusterBar* b, uint64_t* which, 
         : "r"(at), "r"(parity)
         : "memory");
     if (ok || *dead) break;
-    if (clock64() - t0 > kClusterWaitClocks) {
+    if (clock64() - t0 > limit) {
       *dead = 1;
       break;
     }

@@ -176,7 +176,8 @@ class PaperOuter:
                                            _p(self.new), _p(self.scratch), None, None, _sp()), "pgj_paper_oc")
 
     def record(self):
-        """Device view of (steps, change) of the last asynchronous OC update."""
+        """Device view of (steps, change) of the last asynchronous OC update; (-1, NaN) when its blocks waited in
+        vain for each other and ``new`` is unfinished (``step`` raises then)."""
         N = self.n ** 3
         return self.scratch[4 * N + 3:4 * N + 5]
 

@@ -317,6 +317,8 @@ class Server:
             _lib.check(st, "pgj_solve_wait")
         its = max(i.iterations for i in info)
         lineage = isinstance(job.req, Lineage)
+        if lineage and st == _lib.PGJ_OK and math.isnan(float(w.sh[2])):
+            st = _lib.PGJ_ERR_TIMEOUT  # the design update gave up: the lineage keeps its design
         res = StepResult(tag=job.req.tag, kind="design_step" if lineage else "homogenize",
                          step=job.step, n=w.n, C=w.Ch.numpy().copy(),
                          objective=float(w.sh[0]) if lineage else float("nan"), status=st, iterations=its,
@@ -373,7 +375,7 @@ class Server:
                     res = self._finish(w, now)
                     inflight.remove(w)
                     progressed = True
-                    if res.status != 0 and job.precision == "mixed" and self.fallback:
+                    if res.status == _lib.PGJ_ERR_CERTIFICATION and job.precision == "mixed" and self.fallback:
                         # redo in FP64 from the mixed iterate; the design does not advance
                         self.fallbacks += 1
                         redo = _Job(req=job.req, ready=job.ready, lineage=job.lineage, step=job.step,
