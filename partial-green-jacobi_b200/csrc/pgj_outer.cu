@@ -19,9 +19,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
-#include <mutex>
-#include <utility>
 
 namespace pgj {
 
@@ -83,10 +80,11 @@ __global__ void k_grid_wait_selftest(GridBar* bar, double* bounds, unsigned long
 // Taps within kConeR cells: a block of 32 x 8 threads (x fastest) takes a tile of 32 x 8 x kConeZ cells.
 // The tile and its halo sit in shared memory, zero outside the grid (a tap that falls there adds zero),
 // and a thread sums kConeZ cells along z at once: one broadcast read of a tap, then kConeZ reads and
-// multiply-adds without bounds tests. Reads of the tile bound it: 14.7 us a call at n = 64 with 93 taps
+// multiply-adds without bounds tests. Table and tile stay within the 48 KB that a kernel has without setting
+// a limit (384 taps hold every offset of the radius). Reads of the tile bound it: 14.7 us a call at n = 64 with 93 taps
 // (31.4 at n = 96), against 35.2 (76.4) with the neighbours read from global memory one by one. Wider tables (or more than kConeTaps
 // taps) take that loop, kConeTaps taps at a time.
-constexpr int kConeX = 32, kConeY = 8, kConeZ = 4, kConeR = 3, kConeTaps = 512;
+constexpr int kConeX = 32, kConeY = 8, kConeZ = 4, kConeR = 3, kConeTaps = 384;
 struct alignas(16) ConeTap {
   double w;
   long long lin;  // offset of the neighbour in the tile or in the field
@@ -626,6 +624,9 @@ using namespace pgj;
 
 namespace {
 constexpr int kOCBlocks = 296;
+// dynamic shared memory that needs no limit set: 48 KB less the kernels' static arrays
+constexpr size_t kSmemAlways = 48 * 1024 - 384;
+static_assert(sizeof(ConeSmem) <= kSmemAlways, "the cone filter needs no limit set");
 // shared memory of a Study I block up to which the one-launch update is used: two blocks per SM (n = 128 with
 // its own Gaussian takes 49 KB)
 constexpr size_t kS1SmemMax = 100 * 1024;
@@ -635,28 +636,21 @@ int cone_tiles(int n) {
 }
 
 // Blocks of `fn` that are resident together on the current device with `smem` bytes each, at most
-// kOCBlocks; 0 on error. Sets the kernel's shared memory limit. Cached per kernel, device and size.
+// kOCBlocks; 0 on error. Sets the kernel's shared memory limit. Asked on each call: the limit goes with the
+// device's CUDA context when that is replaced (cudaDeviceReset).
 int resident_blocks(const void* fn, int threads, size_t smem) {
-  static std::mutex mutex;
-  static std::map<std::pair<std::pair<const void*, int>, size_t>, int> cache;
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess) return 0;
-  std::lock_guard<std::mutex> lock(mutex);
-  const auto key = std::make_pair(std::make_pair(fn, device), smem);
-  const auto it = cache.find(key);
-  if (it != cache.end()) return it->second;
-  int per = 0, sms = 0;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  int device = 0, per = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess && smem > kSmemAlways)
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kS1SmemMax));
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess) return set_cuda_error(e), 0;
-  return cache[key] = std::min(kOCBlocks, per * sms);
+  return std::min(kOCBlocks, per * sms);
 }
 
 int launch_cone(int n, const int32_t* offsets, const double* weights, int count, const double* x, double* y,
                 cudaStream_t s) {
-  const void* fn = reinterpret_cast<const void*>(&k_cone_filter);
-  if (resident_blocks(fn, kConeX * kConeY, sizeof(ConeSmem)) < 1) return PGJ_ERR_LAUNCH;
   const int tiles = cone_tiles(n);
   k_cone_filter<<<std::min(tiles, 4 * kOCBlocks), kConeBlock, sizeof(ConeSmem), s>>>(n, tiles, offsets, weights, count,
                                                                                     x, y);

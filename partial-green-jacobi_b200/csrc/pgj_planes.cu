@@ -9,9 +9,6 @@
 // 178 / 131 / 123; n = 128 235 / 178 / 216 against 1307.
 #include "pgj_planes.cuh"
 #include <cstring>
-#include <mutex>
-#include <set>
-#include <utility>
 
 namespace pgj {
 
@@ -40,8 +37,6 @@ const Table& table() {
   static const Table t;
   return t;
 }
-std::mutex g_mutex;
-std::set<std::pair<const void*, int>> g_prepared;  // kernel, device
 }  // namespace
 
 const PlaneKernels* planes_find(int n, int prec) {
@@ -56,20 +51,13 @@ bool fused_selectable(int n, int prec) {
   return planes_find(n, prec) && 4 * size_t(n) * nsp * (prec == PGJ_FP32 ? 4 : 8) <= 110 * 1024;
 }
 
-// Shared memory limits of a grid's kernels on the current device.
+// Shared memory limits of a grid's kernels on the current device. Set for every context: they go with the device's
+// CUDA context when that is replaced (cudaDeviceReset).
 int planes_prepare(const PlaneKernels* k) {
-  int device = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return set_cuda_error(e);
-  std::lock_guard<std::mutex> lock(g_mutex);
-  const auto key = std::make_pair(k->fwd, device);
-  if (g_prepared.count(key)) return PGJ_OK;
-  e = cudaFuncSetAttribute(k->fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
+  cudaError_t e = cudaFuncSetAttribute(k->fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k->inv, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k->z, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->zsmem));
-  if (e != cudaSuccess) return set_cuda_error(e);
-  g_prepared.insert(key);
-  return PGJ_OK;
+  return e == cudaSuccess ? PGJ_OK : set_cuda_error(e);
 }
 
 static PlaneArgs plane_args(pgj_ctx* c, int loads) {

@@ -2,9 +2,6 @@
 // device can co-schedule a grid's clusters, and the launch.
 #include "pgj_resident.cuh"
 #include <cstdlib>
-#include <map>
-#include <mutex>
-#include <utility>
 
 namespace pgj {
 
@@ -44,9 +41,6 @@ cudaLaunchConfig_t config(const ResidentKernel& k, int loads, cudaLaunchAttribut
   cfg.numAttrs = 1;
   return cfg;
 }
-
-std::mutex g_mutex;
-std::map<std::pair<const void*, int>, bool> g_fits;  // per kernel and device
 }  // namespace
 
 const ResidentKernel* resident_find(int n, int prec) {
@@ -62,30 +56,24 @@ size_t resident_halo_bytes(int n, int prec) {
 }
 
 // Sets the kernel's launch limits on the current device and asks whether one cluster can be resident
-// there at all (a device partition may have too few SMs in a cluster's reach).
+// there at all (a device partition may have too few SMs in a cluster's reach). Asked for every context: the
+// limits go with the device's CUDA context when that is replaced (cudaDeviceReset).
 const ResidentKernel* resident_prepare(int n, int prec) {
   const char* e = std::getenv("PGJ_RESIDENT");
   if (e && e[0] == '0') return nullptr;
   const ResidentKernel* k = resident_find(n, prec);
-  int device = 0;
-  if (!k || cudaGetDevice(&device) != cudaSuccess) return nullptr;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  const auto key = std::make_pair(k->fn, device);
-  auto it = g_fits.find(key);
-  if (it == g_fits.end()) {
-    cudaError_t err = cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
-    if (err == cudaSuccess && k->cl > 8)
-      err = cudaFuncSetAttribute(k->fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    int clusters = 0;
-    if (err == cudaSuccess) {
-      cudaLaunchAttribute at;
-      const cudaLaunchConfig_t cfg = config(*k, 1, &at, nullptr);
-      err = cudaOccupancyMaxActiveClusters(&clusters, k->fn, &cfg);
-    }
-    if (err != cudaSuccess) cudaGetLastError();  // not launchable here: the separate kernels serve
-    it = g_fits.emplace(key, err == cudaSuccess && clusters >= 1).first;
+  if (!k) return nullptr;
+  cudaError_t err = cudaFuncSetAttribute(k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(k->smem));
+  if (err == cudaSuccess && k->cl > 8)
+    err = cudaFuncSetAttribute(k->fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  int clusters = 0;
+  if (err == cudaSuccess) {
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = config(*k, 1, &at, nullptr);
+    err = cudaOccupancyMaxActiveClusters(&clusters, k->fn, &cfg);
   }
-  return it->second ? k : nullptr;
+  if (err != cudaSuccess) cudaGetLastError();  // not launchable here: the separate kernels serve
+  return err == cudaSuccess && clusters >= 1 ? k : nullptr;
 }
 
 template <typename T>
