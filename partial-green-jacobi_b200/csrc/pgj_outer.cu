@@ -82,23 +82,30 @@ __global__ void k_grid_wait_selftest(GridBar* bar, double* bounds, unsigned long
 // and a thread sums kConeZ cells along z at once: one broadcast read of a tap, then kConeZ reads and
 // multiply-adds without bounds tests. Table and tile stay within the 48 KB that a kernel has without setting
 // a limit (384 taps hold every offset of the radius). Reads of the tile bound it: 14.7 us a call at n = 64 with 93 taps
-// (31.4 at n = 96), against 35.2 (76.4) with the neighbours read from global memory one by one. Wider tables (or more than kConeTaps
-// taps) take that loop, kConeTaps taps at a time.
+// (31.3 at n = 96), against 35.2 (76.4) with the neighbours read from global memory one by one.
+//
+// Farther or longer tables take the general loop, which reads neighbours through the L1, 1, 2 or 4 cells along z per
+// thread, kConeTaps taps at a time. Instructions bound it on large grids (tests, addresses and selects of a tap are
+// shared by a thread's cells), the latency of a group's loads on small ones. us a call, one cell per thread with a branch
+// per tap / four cells one after the other / this loop: 389 taps n = 24 54 / 217 / 35, 64 123 / 281 / 103, 128 647 /
+// 1403 / 543; 4169 taps n = 24 539 / 2235 / 330, 64 1165 / 2710 / 1026.
 constexpr int kConeX = 32, kConeY = 8, kConeZ = 4, kConeR = 3, kConeTaps = 384;
 struct alignas(16) ConeTap {
   double w;
   long long lin;  // offset of the neighbour in the tile or in the field
 };
-struct ConeWide {
-  int dx, dy, dz;
+struct alignas(16) ConeWide {
+  int dx, dy, dz, pad;
+  long long lin;
+  double w;
 };
 constexpr int kConeTile = (kConeX + 2 * kConeR) * (kConeY + 2 * kConeR) * (kConeZ + 2 * kConeR);
-struct ConeSmem {
-  ConeTap taps[kConeTaps];
-  union {
+union ConeSmem {
+  struct {
+    ConeTap taps[kConeTaps];
     double tile[kConeTile];
-    ConeWide wide[kConeTaps];
   };
+  ConeWide wide[kConeTaps];
 };
 
 // Radius of the tap table (max |offset|) if it fits the tile form, else -1; the tile form's tap table is
@@ -131,107 +138,165 @@ __device__ __forceinline__ int cone_stage(ConeSmem& sm, const int32_t* __restric
   return r;
 }
 
-// Filters tile `t` of the field (tiles x fastest, then y, then z); out(cell, value) receives the cells.
-// load(cell) gives the field.
-template <class Load, class Out>
-__device__ __forceinline__ void cone_tile(ConeSmem& sm, int radius, int n, const int32_t* __restrict__ offsets,
-                                          const double* __restrict__ weights, int count, int t, Load load, Out out) {
+// Tiles of `depth` planes along z.
+__host__ __device__ inline int cone_tiles(int n, int depth) {
+  return ((n + kConeX - 1) / kConeX) * ((n + kConeY - 1) / kConeY) * ((n + depth - 1) / depth);
+}
+
+// General loop over tile `t` (tiles x fastest, then y, then z) of K planes, K cells along z per thread: any table, taps
+// outside the grid skipped. The cells share a tap's reads and its tests in the plane, and the loads of U taps are in
+// flight together, without branches: where a tap falls outside, a cell of the thread's own stands in and the sum is left
+// as it was.
+template <int K, class Out>
+__device__ __forceinline__ void cone_general(ConeSmem& sm, int n, const int32_t* __restrict__ offsets,
+                                             const double* __restrict__ weights, int count, int t, const double* src,
+                                             Out out) {
+  const int nx = (n + kConeX - 1) / kConeX, ny = (n + kConeY - 1) / kConeY;
+  const int bz = t / (nx * ny), rem = t - bz * nx * ny, by = rem / nx, bx = rem - by * nx;
+  const int cx = bx * kConeX + threadIdx.x, cy = by * kConeY + threadIdx.y, cz = bz * K;
+  constexpr int U = K == 4 ? 2 : 4;
+  static_assert(kConeTaps % U == 0, "chunks are whole groups");
+  const bool inside = cx < n && cy < n;
+  const unsigned un = unsigned(n);
+  const size_t plane = size_t(n) * n;
+  const size_t at0 = (size_t(cz) * n + cy) * n + cx;
+  const double* cell = src + at0;
+  double acc[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) acc[k] = 0.0;
+  for (int first = 0; first < count; first += kConeTaps) {
+    const int m = min(kConeTaps, count - first), groups = (m + U - 1) / U;
+    __syncthreads();  // the previous chunk has been read
+    for (int j = flat_tid(); j < groups * U; j += kConeX * kConeY) {
+      ConeWide w = {n, n, n, 0, 0, 0.0};  // fills up the last group: outside from any cell
+      if (j < m) {
+        const int at = 3 * (first + j);
+        w.dx = offsets[at]; w.dy = offsets[at + 1]; w.dz = offsets[at + 2];
+        w.lin = (static_cast<long long>(w.dz) * n + w.dy) * n + w.dx;
+        w.w = weights[first + j];
+      }
+      sm.wide[j] = w;
+    }
+    __syncthreads();
+    if (!inside) continue;
+#pragma unroll 1
+    for (int g = 0; g < groups; ++g) {
+      double w[U], v[U][K];
+      bool in[U][K];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const ConeWide& tap = sm.wide[g * U + u];
+        w[u] = tap.w;
+        const bool xy = unsigned(cx) + unsigned(tap.dx) < un && unsigned(cy) + unsigned(tap.dy) < un;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          in[u][k] = xy && unsigned(cz + k) + unsigned(tap.dz) < un;
+          v[u][k] = cell[in[u][k] ? tap.lin + static_cast<long long>(k * plane) : 0];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          acc[k] = in[u][k] ? fma(w[u], v[u][k], acc[k]) : acc[k];
+    }
+  }
+  if (inside)
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (cz + k < n) out(at0 + k * plane, acc[k]);
+}
+
+// Tiled form over tile `t` of kConeZ planes; out(cell, value) receives the cells.
+template <class Out>
+__device__ __forceinline__ void cone_tile(ConeSmem& sm, int radius, int n, int count, int t, const double* src, Out out) {
   const int nx = (n + kConeX - 1) / kConeX, ny = (n + kConeY - 1) / kConeY;
   const int bz = t / (nx * ny), rem = t - bz * nx * ny, by = rem / nx, bx = rem - by * nx;
   const int lx = threadIdx.x, ly = threadIdx.y;
   const int x0 = bx * kConeX, y0 = by * kConeY, z0 = bz * kConeZ;
   const int cx = x0 + lx, cy = y0 + ly;
-  const bool inside = cx < n && cy < n;
   double acc[kConeZ];
 #pragma unroll
   for (int k = 0; k < kConeZ; ++k) acc[k] = 0.0;
-  if (radius >= 0) {
-    const int px = kConeX + 2 * radius, py = kConeY + 2 * radius, pz = kConeZ + 2 * radius;
-    __syncthreads();  // the previous tile has been read
-    // a thread fills whole z columns of the tile, all loads of a column in flight together
-    for (int p = flat_tid(); p < px * py; p += kConeX * kConeY) {
-      const int y = p / px, x = p - y * px, gx = x0 + x - radius, gy = y0 + y - radius;
-      const bool in = unsigned(gx) < unsigned(n) && unsigned(gy) < unsigned(n);
-      double v[kConeZ + 2 * kConeR];
+  const int px = kConeX + 2 * radius, py = kConeY + 2 * radius, pz = kConeZ + 2 * radius;
+  __syncthreads();  // the previous tile has been read
+  // a thread fills whole z columns of the tile, all loads of a column in flight together
+  for (int p = flat_tid(); p < px * py; p += kConeX * kConeY) {
+    const int y = p / px, x = p - y * px, gx = x0 + x - radius, gy = y0 + y - radius;
+    const bool in = unsigned(gx) < unsigned(n) && unsigned(gy) < unsigned(n);
+    double v[kConeZ + 2 * kConeR];
 #pragma unroll
-      for (int z = 0; z < kConeZ + 2 * kConeR; ++z) {
-        const int gz = z0 + z - radius;
-        v[z] = in && z < pz && unsigned(gz) < unsigned(n) ? load((size_t(gz) * n + gy) * n + gx) : 0.0;
-      }
-#pragma unroll
-      for (int z = 0; z < kConeZ + 2 * kConeR; ++z)
-        if (z < pz) sm.tile[z * px * py + p] = v[z];
+    for (int z = 0; z < kConeZ + 2 * kConeR; ++z) {
+      const int gz = z0 + z - radius;
+      v[z] = in && z < pz && unsigned(gz) < unsigned(n) ? __ldcg(src + (size_t(gz) * n + gy) * n + gx) : 0.0;
     }
-    __syncthreads();
-    const double* at = sm.tile + (radius * py + ly + radius) * px + lx + radius;
-    const int pl = px * py;
-    // eight taps' reads are in flight before their multiply-adds (a tap at a time waits out two shared
-    // memory latencies per tap)
-    constexpr int U = 8;
-    int j = 0;
-    for (; j + U <= count; j += U) {
-      double w[U], v[U][kConeZ];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const ConeTap tap = sm.taps[j + u];
-        w[u] = tap.w;
-        const double* p = at + int(tap.lin);
-#pragma unroll
-        for (int k = 0; k < kConeZ; ++k) v[u][k] = p[k * pl];
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int k = 0; k < kConeZ; ++k) acc[k] += w[u] * v[u][k];
-    }
-    for (; j < count; ++j) {
-      const double w = sm.taps[j].w;
-      const double* p = at + int(sm.taps[j].lin);
-#pragma unroll
-      for (int k = 0; k < kConeZ; ++k) acc[k] += w * p[k * pl];
-    }
-  } else {
-    const int tid = flat_tid();
-    const unsigned un = unsigned(n);
-    for (int first = 0; first < count; first += kConeTaps) {
-      const int m = min(kConeTaps, count - first);
-      __syncthreads();  // the previous chunk has been read
-      for (int j = tid; j < m; j += kConeX * kConeY) {
-        const int dx = offsets[3 * (first + j)], dy = offsets[3 * (first + j) + 1], dz = offsets[3 * (first + j) + 2];
-        sm.wide[j].dx = dx;
-        sm.wide[j].dy = dy;
-        sm.wide[j].dz = dz;
-        sm.taps[j].w = weights[first + j];
-        sm.taps[j].lin = (static_cast<long long>(dz) * n + dy) * n + dx;
-      }
-      __syncthreads();
-      if (!inside) continue;
-#pragma unroll
-      for (int k = 0; k < kConeZ; ++k) {
-        const int cz = z0 + k;
-        if (cz >= n) break;
-        const long long cell = (static_cast<long long>(cz) * n + cy) * n + cx;
-        for (int j = 0; j < m; ++j)
-          if (unsigned(cx + sm.wide[j].dx) < un && unsigned(cy + sm.wide[j].dy) < un && unsigned(cz + sm.wide[j].dz) < un)
-            acc[k] += sm.taps[j].w * load(size_t(cell + sm.taps[j].lin));
-      }
-    }
+    for (int z = 0; z < kConeZ + 2 * kConeR; ++z)
+      if (z < pz) sm.tile[z * px * py + p] = v[z];
   }
-  if (inside)
+  __syncthreads();
+  const double* at = sm.tile + (radius * py + ly + radius) * px + lx + radius;
+  const int pl = px * py;
+  // eight taps' reads are in flight before their multiply-adds (a tap at a time waits out two shared
+  // memory latencies per tap)
+  constexpr int U = 8;
+  int j = 0;
+  for (; j + U <= count; j += U) {
+    double w[U], v[U][kConeZ];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const ConeTap tap = sm.taps[j + u];
+      w[u] = tap.w;
+      const double* p = at + int(tap.lin);
+#pragma unroll
+      for (int k = 0; k < kConeZ; ++k) v[u][k] = p[k * pl];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < kConeZ; ++k) acc[k] += w[u] * v[u][k];
+  }
+  for (; j < count; ++j) {
+    const double w = sm.taps[j].w;
+    const double* p = at + int(sm.taps[j].lin);
+#pragma unroll
+    for (int k = 0; k < kConeZ; ++k) acc[k] += w * p[k * pl];
+  }
+  if (cx < n && cy < n)
 #pragma unroll
     for (int k = 0; k < kConeZ; ++k)
       if (z0 + k < n) out((size_t(z0 + k) * n + cy) * n + cx, acc[k]);
 }
 
-__global__ void __launch_bounds__(kConeX * kConeY) k_cone_filter(int n, int tiles, const int32_t* __restrict__ offsets,
+// Calls body(filter) for every tile of the block; filter(src, out) filters the tile of the field `src`, out(cell, value)
+// receives its cells.
+template <class Body>
+__device__ __forceinline__ void cone_fields(ConeSmem& sm, int radius, int n, const int32_t* __restrict__ offsets,
+                                            const double* __restrict__ weights, int count, Body body) {
+  const int t = blockIdx.x, nblk = gridDim.x;
+  if (radius >= 0) {
+    for (int i = t; i < cone_tiles(n, kConeZ); i += nblk)
+      body([&](const double* src, auto out) { cone_tile(sm, radius, n, count, i, src, out); });
+  } else if (cone_tiles(n, 1) <= nblk) {  // as few planes a tile as give every block one
+    if (t < cone_tiles(n, 1))
+      body([&](const double* src, auto out) { cone_general<1>(sm, n, offsets, weights, count, t, src, out); });
+  } else if (cone_tiles(n, 2) <= nblk) {
+    if (t < cone_tiles(n, 2))
+      body([&](const double* src, auto out) { cone_general<2>(sm, n, offsets, weights, count, t, src, out); });
+  } else {
+    for (int i = t; i < cone_tiles(n, kConeZ); i += nblk)
+      body([&](const double* src, auto out) { cone_general<kConeZ>(sm, n, offsets, weights, count, i, src, out); });
+  }
+}
+
+__global__ void __launch_bounds__(kConeX * kConeY) k_cone_filter(int n, const int32_t* __restrict__ offsets,
                                                                  const double* __restrict__ weights, int count,
                                                                  const double* __restrict__ x, double* __restrict__ y) {
   extern __shared__ __align__(16) unsigned char raw[];
   ConeSmem& sm = *reinterpret_cast<ConeSmem*>(raw);
   const int radius = cone_stage(sm, offsets, weights, count);
-  for (int t = blockIdx.x; t < tiles; t += gridDim.x)
-    cone_tile(sm, radius, n, offsets, weights, count, t, [&](size_t i) { return x[i]; },
-              [&](size_t i, double v) { y[i] = v; });
+  cone_fields(sm, radius, n, offsets, weights, count,
+              [&](auto filter) { filter(x, [&](size_t i, double v) { y[i] = v; }); });
 }
 
 // te = tanh(beta eta), den = te + tanh(beta (1 - eta))
@@ -257,14 +322,14 @@ __global__ void k_paper_project(size_t N, const double* __restrict__ t, const do
 
 // Bisection record shared with the callers: lo, hi, continue flag, steps taken, max |xnew - x|.
 struct OCArgs {
-  int n, tiles;
+  int n;
   const int32_t* offsets;  // paper: cone taps
   const double* weights;   // cone weights, or the Gaussian's 2 radius + 1
   int count;               // taps, or the Gaussian's radius
   const double *x, *ph, *dp, *hs, *energy;
   double volume, beta, eta, emin, move, exponent, floor_;
   double* xnew;
-  double *f0, *f1, *f2, *f3;  // ratio, dv, temporaries
+  double *f0, *f2, *f3;  // ratio, temporaries
   double* bounds;
   GridBar* bar;
   double* partials;
@@ -289,6 +354,8 @@ __device__ __forceinline__ void grid_max(double m, double* out) {
     atomicMax(reinterpret_cast<unsigned long long*>(out), static_cast<unsigned long long>(__double_as_longlong(m)));
 }
 
+// Fields that other blocks wrote are read after a grid barrier only, whose acquire orders plain loads too.
+//
 // Damped OC update of the paper's chain (reproduction.py:92-118): filtered sensitivities, ratio, and the
 // bisection of the multiplier. Per step: candidate design; barrier; cone filter of it, projection, volume
 // partials; barrier.
@@ -309,18 +376,10 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
   }
   if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
   const double dN = double(N);
-  for (int t = blockIdx.x; t < A.tiles; t += gridDim.x) {
-    double g[kConeZ];
-    int k = 0;
-    cone_tile(sm, radius, n, A.offsets, A.weights, A.count, t, [&](size_t i) { return __ldcg(A.f2 + i); },
-              [&](size_t, double v) { g[k++] = v; });
-    k = 0;
-    cone_tile(sm, radius, n, A.offsets, A.weights, A.count, t, [&](size_t i) { return __ldcg(A.f3 + i); },
-              [&](size_t i, double v) {
-                A.f0[i] = -(g[k++] / dN) / v;
-                A.f1[i] = v;
-              });
-  }
+  cone_fields(sm, radius, n, A.offsets, A.weights, A.count, [&](auto filter) {
+    filter(A.f2, [&](size_t i, double v) { A.f0[i] = v; });
+    filter(A.f3, [&](size_t i, double v) { A.f0[i] = -(A.f0[i] / dN) / v; });
+  });
   if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
   const double te = tanh(A.beta * A.eta), den = te + tanh(A.beta * (1 - A.eta));
   double lo = 0.0, hi = 1e9, steps = 0.0;
@@ -334,13 +393,13 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
     }
     if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
     double acc[1] = {0.0};
-    for (int t = blockIdx.x; t < A.tiles; t += gridDim.x)
-      cone_tile(sm, radius, n, A.offsets, A.weights, A.count, t, [&](size_t i) { return __ldcg(A.xnew + i); },
-                [&](size_t i, double v) {
-                  double p, d, a;
-                  paper_phys(v, A.hs[i], A.beta, A.eta, A.emin, te, den, p, d, a);
-                  acc[0] += p;
-                });
+    cone_fields(sm, radius, n, A.offsets, A.weights, A.count, [&](auto filter) {
+      filter(A.xnew, [&](size_t i, double v) {
+        double p, d, a;
+        paper_phys(v, A.hs[i], A.beta, A.eta, A.emin, te, den, p, d, a);
+        acc[0] += p;
+      });
+    });
     block_sum<1>(acc, red);
     if (tid == 0) A.partials[blockIdx.x] = acc[0];
     if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
@@ -631,8 +690,10 @@ static_assert(sizeof(ConeSmem) <= kSmemAlways, "the cone filter needs no limit s
 // its own Gaussian takes 49 KB)
 constexpr size_t kS1SmemMax = 100 * 1024;
 const dim3 kConeBlock(kConeX, kConeY);
-int cone_tiles(int n) {
-  return ((n + kConeX - 1) / kConeX) * ((n + kConeY - 1) / kConeY) * ((n + kConeZ - 1) / kConeZ);
+// Blocks that filter a field, at most `most`: one per tile of the tiled form; tables too long for it take up to one per
+// plane of a tile.
+int cone_blocks(int n, int count, int most) {
+  return std::min(cone_tiles(n, count > kConeTaps ? 1 : kConeZ), most);
 }
 
 // Blocks of `fn` that are resident together on the current device with `smem` bytes each, at most
@@ -651,9 +712,7 @@ int resident_blocks(const void* fn, int threads, size_t smem) {
 
 int launch_cone(int n, const int32_t* offsets, const double* weights, int count, const double* x, double* y,
                 cudaStream_t s) {
-  const int tiles = cone_tiles(n);
-  k_cone_filter<<<std::min(tiles, 4 * kOCBlocks), kConeBlock, sizeof(ConeSmem), s>>>(n, tiles, offsets, weights, count,
-                                                                                    x, y);
+  k_cone_filter<<<cone_blocks(n, count, 4 * kOCBlocks), kConeBlock, sizeof(ConeSmem), s>>>(n, offsets, weights, count, x, y);
   return check_launch();
 }
 
@@ -745,15 +804,15 @@ int pgj_paper_oc(int n, const int32_t* offsets, const double* weights, int count
   cudaError_t e = cudaMemsetAsync(w.bounds, 0, 16 * sizeof(double), s);
   if (e != cudaSuccess) return set_cuda_error(e);
   OCArgs A = {};
-  A.n = n; A.tiles = cone_tiles(n);
+  A.n = n;
   A.offsets = offsets; A.weights = weights; A.count = count;
   A.x = x; A.ph = ph; A.dp = dp; A.hs = hs; A.energy = energy;
   A.volume = volume; A.beta = beta; A.eta = eta; A.emin = emin; A.move = move; A.exponent = exponent; A.floor_ = floor_;
   A.xnew = xnew;
-  A.f0 = w.f0; A.f1 = w.f1; A.f2 = w.f2; A.f3 = w.f3;
+  A.f0 = w.f0; A.f2 = w.f2; A.f3 = w.f3;
   A.bounds = w.bounds; A.bar = reinterpret_cast<GridBar*>(w.ticket); A.partials = w.partials;
-  const int st = launch_oc(reinterpret_cast<const void*>(&k_paper_oc), kConeBlock, sizeof(ConeSmem),
-                           std::max<size_t>(A.tiles, (N + kConeX * kConeY - 1) / (kConeX * kConeY)), A, s);
+  const size_t work = std::max<size_t>(cone_blocks(n, count, kOCBlocks), (N + kConeX * kConeY - 1) / (kConeX * kConeY));
+  const int st = launch_oc(reinterpret_cast<const void*>(&k_paper_oc), kConeBlock, sizeof(ConeSmem), work, A, s);
   if (st) return st;
   if (!steps && !change) return PGJ_OK;  // enqueue only: the record stays in scratch[4N + 3 .. 4N + 4]
   return read_record(w, steps, change, s);

@@ -1,5 +1,6 @@
 """The cone filter on tap tables that PaperOuter does not build: offsets far outside the grid, anisotropic and long
-tables, and weights that are not finite, against the sum over the taps whose neighbour lies inside the grid.
+tables, and weights that are not finite, against the sum over the taps whose neighbour lies inside the grid; and design
+updates with wide filters, at grids of each tile depth of the general loop (bounds as in test_outer_updates.py).
 
 Taps are summed in table order with one fused multiply-add each; the reference sums products, so a cell's difference is
 below (taps + 1) x 2^-53 times the sum of |w x|. Cells that a non-finite weight reaches agree in kind."""
@@ -36,7 +37,7 @@ def tables():
     yield "nan", [[0, 0, 0], [0, 0, 3]], [1.0, np.nan]
 
 
-@pytest.mark.parametrize("n", [2, 5, 33])
+@pytest.mark.parametrize("n", [2, 5, 33, 64])
 def test_general_tables(pkg, n):
     x = np.random.default_rng(n).uniform(0.1, 1.0, (n, n, n))
     xd = torch.tensor(x, device="cuda")
@@ -53,3 +54,20 @@ def test_general_tables(pkg, n):
         assert np.array_equal(np.isfinite(got), fin), name
         assert np.array_equal(np.isposinf(got), np.isposinf(want)), name
         assert np.all(np.abs(got - want)[fin] <= (len(weights) + 1) * 2.0 ** -53 * size[fin]), name
+
+
+@pytest.mark.parametrize("n,rmin", [(9, 4.2), (40, 4.6), (50, 4.6)])
+def test_paper_update_with_a_wide_filter(pkg, oracle, n, rmin):
+    rng = np.random.default_rng(n)
+    x, e = rng.uniform(0.05, 0.95, (n, n, n)), rng.uniform(0.1, 2.0, (n, n, n))
+    po = pkg.PaperOuter(n, 0.3, rmin=rmin, emin=1e-6)
+    po.set_initial(x)
+    po.evaluate()
+    hs, t = oracle.cone_filter(np.ones_like(x), rmin), oracle.cone_filter(x, rmin)
+    assert np.abs(po.t.cpu().numpy() / t - 1).max() < 1e-13
+    ph, dp, _ = oracle.paper_physical(t, hs, emin=1e-6)
+    po.step(torch.tensor(-e, device="cuda"))
+    new, steps, change = oracle.paper_oc(x, -e, ph, dp, hs, rmin, 0.3, emin=1e-6)
+    assert po.steps == steps
+    assert np.abs(po.new.cpu().numpy() - new).max() < 1e-12
+    assert abs(float(po.change) - change) < 1e-12
