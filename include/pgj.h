@@ -195,18 +195,20 @@ int pgj_profile_iteration(pgj_ctx* ctx, int loads, const double* macros, int rep
  * update), or on small grids one resident kernel for all of them; 0: the operator, the two vector
  * updates and the five Green passes as separate kernels. 1 is the default where two transform planes fit
  * in an SM's shared memory (n <= 80 in FP64, 108 in FP32); pgj_set_fused_iteration returns
- * PGJ_ERR_UNSUPPORTED for 1 on other grids. Those report 0, and the library runs the four-kernel form
- * there too as long as one plane pair fits (n <= 108 in FP64, 128 in FP32), unless 0 is set explicitly. */
+ * PGJ_ERR_UNSUPPORTED for 1 on other grids. Those have no choice: they report 0, writing 0 changes
+ * nothing, and they run the four-kernel form as long as one plane pair fits (n <= 108 in FP64, 128 in
+ * FP32; unless PGJ_UNFUSED was in the environment when the context was created), the separate kernels
+ * beyond. pgj_tile_shapes and pgj_tile_config report the set that runs. */
 int pgj_fused_iteration(pgj_ctx* ctx);
 int pgj_set_fused_iteration(pgj_ctx* ctx, int on);
 
 /* Tile shapes the context's autotuners picked (no reference counterpart): out[0] operator rows per
  * block, out[1] operator z-planes per block, out[2] rows per x-pass block, out[3] / out[4] kx columns
- * per y / z-pass block, out[5] fused iteration flag. */
+ * per y / z-pass block, out[5] 1 when the four-kernel iteration (or the resident kernel) runs. */
 int pgj_tile_shapes(pgj_ctx* ctx, int* out);
 /* The context's tile configuration (no reference counterpart): out[0..3]
  * operator rows per block, z-planes per block, 0, blocks per SM; out[4..6] requested FFT
- * rows per x block, y chunks, z chunks; out[7] fused iteration flag; out[8] where the FFT tiles came from
+ * rows per x block, y chunks, z chunks; out[7] as out[5] of pgj_tile_shapes; out[8] where the FFT tiles came from
  * (0 timed at creation, 1 the tile table built in, 2 environment override). */
 int pgj_tile_config(pgj_ctx* ctx, int* out);
 

@@ -791,7 +791,7 @@ int pgj_tile_shapes(pgj_ctx* c, int* out) {
   if (!c || !out) return PGJ_ERR_ARGUMENT;
   const StencilGeom& g = c->prec == PGJ_FP32 ? c->geo32 : c->geo64;
   out[0] = g.ty; out[1] = g.zc; out[2] = c->fg.rb; out[3] = c->fg.kcy; out[4] = c->fg.kcz;
-  out[5] = c->fused;
+  out[5] = c->four;
   return PGJ_OK;
 }
 
@@ -800,13 +800,14 @@ int pgj_tile_config(pgj_ctx* c, int* out) {
   const StencilGeom& g = c->prec == PGJ_FP32 ? c->geo32 : c->geo64;
   out[0] = g.ty; out[1] = g.zc; out[2] = 0; out[3] = g.occ;
   out[4] = c->fft_req[0]; out[5] = c->fft_req[1]; out[6] = c->fft_req[2];
-  out[7] = c->fused; out[8] = c->tile_source;
+  out[7] = c->four; out[8] = c->tile_source;
   return PGJ_OK;
 }
 
 int pgj_set_fused_iteration(pgj_ctx* c, int on) {
   if (!c || (on != 0 && on != 1)) return PGJ_ERR_ARGUMENT;
-  if (on && !fused_selectable(c->n, c->prec)) return PGJ_ERR_UNSUPPORTED;
+  // without a choice the reported 0 may be written back: the context keeps the kernel set it has
+  if (!fused_selectable(c->n, c->prec)) return on ? PGJ_ERR_UNSUPPORTED : PGJ_OK;
   c->fused = c->four = on;
   c->graphs->loads = 0;  // rebuild the solve graphs with the other kernel set
   c->graphs->attempt_loads = 0;

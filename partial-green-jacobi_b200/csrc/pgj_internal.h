@@ -202,7 +202,7 @@ const PlaneKernels* planes_find(int n, int prec);
 int planes_prepare(const PlaneKernels* k);
 // grids on which pgj_set_fused_iteration selects between the two kernel sets: two planes of transform
 // buffers per SM (up to n = 80 in FP64, 108 in FP32). Larger grids whose plane pair fits one block per SM run
-// the plane kernels as well, but report and accept only 0.
+// the plane kernels as well, without a choice: they report 0, and writing that back changes nothing.
 bool fused_selectable(int n, int prec);
 int launch_planes_fwd(pgj_ctx* c, int loads, int mode, cudaStream_t s, cudaGraphConditionalHandle hif = 0);
 int launch_planes_z(pgj_ctx* c, int loads, bool init, cudaStream_t s);

@@ -247,7 +247,8 @@ class Operator:
 
     @property
     def fused_iteration(self) -> bool:
-        """True when one PCG iteration runs as four kernels (updates fused with the transforms)."""
+        """True when the four-kernel iteration (updates fused with the transforms; on small grids the resident
+        kernel) is selected on a grid that has the choice. ``tile_shapes()["fused"]`` is what runs."""
         return bool(_lib.lib().pgj_fused_iteration(self._ctx))
 
     def set_fused_iteration(self, on: bool) -> None:
