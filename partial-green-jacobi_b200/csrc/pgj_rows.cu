@@ -1,5 +1,6 @@
 // Launch of the operator (pgj_rows.cuh): tile choice and instantiations.
 #include "pgj_rows.cuh"
+#include <algorithm>
 
 namespace pgj {
 
@@ -8,6 +9,11 @@ namespace {
 // 250 registers in FP64 (128 would spill: 2 to 3 times slower) and 150 in FP32, where 256 threads leave latency
 // uncovered on large grids (n = 96 93 against 88 us, 128 227 against 205) and 512 spill (n = 64 36 against 27).
 constexpr int kThr64 = 256, kThr32 = 384;
+// Blocks per SM at most: in FP64 the exchange buffers (49 KB whatever the block's size) leave room for four; in FP32
+// for six, and the recurrence's instance has registers for five blocks of two warps.
+// Counting eight, as the threads alone would allow, took shapes with a second, nearly empty wave: recurrence operator of
+// six loads n = 24 18.5 us FP64, 14.4 mixed (14.3, 12.3 now), n = 30 20.5, 16.4 (14.4, 12.3), n = 32 mixed 15.3 (12.3).
+constexpr int kPer64 = 4, kPer32 = 5;
 
 template <typename T, int MODE, typename R, bool COMP, bool VEC>
 struct Rows {
@@ -35,7 +41,8 @@ StencilGeom rows_geom(int n, int lpd, bool wide) {
   double top = -1.0;
   for (int ty = 1; ty <= n && nh * (ty + 1) <= most; ++ty) {
     const int tiles = (n + ty - 1) / ty, warps = (nh * (ty + 1) + 31) / 32;
-    const int per = most / 32 / warps < 8 ? most / 32 / warps : 8;  // blocks per SM
+    // blocks per SM: by threads (registers), at most kPer64 or kPer32
+    const int per = std::min(most / 32 / warps, wide ? kPer64 : kPer32);
     const double rows = double(n) * nh / (double(tiles) * warps * 32) * double(per * warps * 32) / most;
     for (int nch = 1; nch <= (n / 4 > 1 ? n / 4 : 1); ++nch) {
       const int zc = (n + nch - 1) / nch, chunks = (n + zc - 1) / zc;
