@@ -329,7 +329,7 @@ struct OCArgs {
   const double *x, *ph, *dp, *hs, *energy;
   double volume, beta, eta, emin, move, exponent, floor_;
   double* xnew;
-  double *f0, *f2, *f3;  // ratio, temporaries
+  double *f0, *f1, *f2, *f3;  // ratio, dv (both left to the caller: g = -ratio dv), temporaries
   double* bounds;
   GridBar* bar;
   double* partials;
@@ -378,7 +378,10 @@ __global__ void __launch_bounds__(kConeX * kConeY) k_paper_oc(const OCArgs A) {
   const double dN = double(N);
   cone_fields(sm, radius, n, A.offsets, A.weights, A.count, [&](auto filter) {
     filter(A.f2, [&](size_t i, double v) { A.f0[i] = v; });
-    filter(A.f3, [&](size_t i, double v) { A.f0[i] = -(A.f0[i] / dN) / v; });
+    filter(A.f3, [&](size_t i, double v) {
+      A.f0[i] = -(A.f0[i] / dN) / v;
+      A.f1[i] = v;
+    });
   });
   if (!grid_barrier(A.bar, target)) return oc_gave_up(A.bounds);
   const double te = tanh(A.beta * A.eta), den = te + tanh(A.beta * (1 - A.eta));
@@ -809,7 +812,7 @@ int pgj_paper_oc(int n, const int32_t* offsets, const double* weights, int count
   A.x = x; A.ph = ph; A.dp = dp; A.hs = hs; A.energy = energy;
   A.volume = volume; A.beta = beta; A.eta = eta; A.emin = emin; A.move = move; A.exponent = exponent; A.floor_ = floor_;
   A.xnew = xnew;
-  A.f0 = w.f0; A.f2 = w.f2; A.f3 = w.f3;
+  A.f0 = w.f0; A.f1 = w.f1; A.f2 = w.f2; A.f3 = w.f3;
   A.bounds = w.bounds; A.bar = reinterpret_cast<GridBar*>(w.ticket); A.partials = w.partials;
   const size_t work = std::max<size_t>(cone_blocks(n, count, kOCBlocks), (N + kConeX * kConeY - 1) / (kConeX * kConeY));
   const int st = launch_oc(reinterpret_cast<const void*>(&k_paper_oc), kConeBlock, sizeof(ConeSmem), work, A, s);
