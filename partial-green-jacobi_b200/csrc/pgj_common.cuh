@@ -19,37 +19,17 @@ constexpr int kMaxStages = 8;
 
 __host__ __device__ __forceinline__ int wrapi(int x, int n) { return x < 0 ? x + n : (x >= n ? x - n : x); }
 
-// --------------------------------------------------------------------------- TMA bulk copies
+// --------------------------------------------------------------------------- mbarriers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-// --- TMA (bulk async copy) staging: one elected thread copies whole rows into shared memory and
-// the block waits on an mbarrier whose transaction count is the plane's byte size.
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void tma_row(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-// Bulk store shared -> global (the async proxy reads shared memory; make generic writes visible first
-// with fence_proxy_async() and a block barrier, and wait for the reads before the buffer is reused
-// or the block exits).
-__device__ __forceinline__ void tma_store_row(void* gdst, const void* ssrc, unsigned bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(gdst), "r"(smem_u32(ssrc)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
 
 // --------------------------------------------------------------------------- fast division
 // Quotient of a non-negative int below 2^31 by a fixed divisor d with one multiply-high and a
@@ -85,10 +65,6 @@ template <typename C> __device__ __forceinline__ C csub(C a, C b) { C c; c.x = a
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   C c; c.x = a.x * b.x - a.y * b.y; c.y = a.x * b.y + a.y * b.x; return c;
 }
-// a * conj(b)
-template <typename C> __device__ __forceinline__ C cmulc(C a, C b) {
-  C c; c.x = a.x * b.x + a.y * b.y; c.y = a.y * b.x - a.x * b.y; return c;
-}
 template <typename C> __device__ __forceinline__ C cconj(C a) { a.y = -a.y; return a; }
 // FP32 complex arithmetic as packed FP32 operations (two results per instruction on sm_100);
 // adds and subtracts round exactly like their scalar forms
@@ -104,7 +80,6 @@ template <> __device__ __forceinline__ float2 cmul<float2>(float2 a, float2 b) {
 template <typename C> __device__ __forceinline__ C cmul_mi(C a, bool inv) {
   C c; if (inv) { c.x = -a.y; c.y = a.x; } else { c.x = a.y; c.y = -a.x; } return c;
 }
-template <typename C, typename T> __device__ __forceinline__ C cscale(C a, T s) { a.x *= s; a.y *= s; return a; }
 
 // --------------------------------------------------------------------------- batched copies
 // for (i = tid; i < count; i += nthr) st(i, ld(i)), with UNR loads issued before their stores so a
@@ -281,28 +256,6 @@ __host__ __device__ __forceinline__ void element_modal(const T (&Q)[8][3], T A, 
   const T k7 = A * T(k.k7);
   P[7][0] = k7 * Q[7][0]; P[7][1] = k7 * Q[7][1]; P[7][2] = k7 * Q[7][2];
   P[0][0] = T(0); P[0][1] = T(0); P[0][2] = T(0);
-}
-
-// 8 nodal values (b = bx + 2by + 4bz) -> modal Q[m]; all 8 modes.
-template <typename T>
-__host__ __device__ __forceinline__ void hadamard8(const T (&v)[8][3], T (&Q)[8][3]) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    T s[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s[i] = v[i][c];
-    // x level (bit 0)
-#pragma unroll
-    for (int i = 0; i < 8; i += 2) { T a = s[i], b = s[i + 1]; s[i] = b + a; s[i + 1] = b - a; }
-    // y level (bit 1)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) if (!(i & 2)) { T a = s[i], b = s[i + 2]; s[i] = b + a; s[i + 2] = b - a; }
-    // z level (bit 2)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { T a = s[i], b = s[i + 4]; s[i] = b + a; s[i + 4] = b - a; }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) Q[i][c] = s[i];
-  }
 }
 
 }  // namespace pgj

@@ -29,7 +29,7 @@ struct Graphs {
   int attempt_mode = -1;
   double inner_rtol = 0.0;
   cudaGraphExec_t cert = nullptr;
-  cudaGraphExec_t attempt = nullptr;  // FP64: init + PCG loop + certify; mixed: one refinement sweep
+  cudaGraphExec_t attempt = nullptr;  // one refinement sweep
   cudaGraphExec_t solve = nullptr;    // whole certified solve with device-side restarts
   double rtol = 0.0;
   int mode = -1;
@@ -692,9 +692,9 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
     const int st = pgj_solve_async(c, loads, macros, rtol, u, stream);
     return st ? st : pgj_solve_wait(c, info, stream);
   }
+  // restarted refinement sweeps
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t N3 = 3 * size_t(c->N);
-  const bool mixed = c->prec == PGJ_FP32 && c->mixed_mode == 1;  // restarted refinement sweeps
   c->scal = c->scal_out;
   int st = stage_macros(c, loads, macros, s);
   if (!st) st = launch_rhs(c, loads, c->macros, c->f, s);
@@ -708,7 +708,7 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
   if ((e = cudaGraphLaunch(c->graphs->cert, s)) != cudaSuccess) return set_cuda_error(e);
   std::vector<LoadScalars> h(loads);
   std::vector<int> ok(loads, 0);
-  int restarts = 0, sweeps = 0;
+  int sweeps = 0;
   int body[4] = {0, 0, 0, 0};
   long long launches = 2 + 3;  // rhs + norms, initial certification
   bool capped_by_bound = false;
@@ -725,38 +725,21 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
       ok[l] = std::isfinite(h[l].absolute) && h[l].absolute <= thr && h[l].bad == 0;
       all = all && ok[l];
       anybad = anybad || h[l].bad;
-      const int its = mixed ? h[l].total_iterations : h[l].iterations;
-      capped = capped || (!ok[l] && its >= c->cap);
+      capped = capped || (!ok[l] && h[l].total_iterations >= c->cap);
     }
   };
-  if (mixed) {
-    // one FP32 inner solve per sweep inside FP64 iterative refinement
-    if ((e = read_state(false)) != cudaSuccess) return set_cuda_error(e);
-    for (;;) {
-      bool all, anybad, capped;
-      evaluate(all, anybad, capped);
-      if (all || anybad || capped || sweeps >= kMaxSweeps) break;
-      if ((e = cudaGraphLaunch(c->graphs->attempt, s)) != cudaSuccess) return set_cuda_error(e);
-      ++sweeps;
-      if ((e = read_state(true)) != cudaSuccess) return set_cuda_error(e);
-      // sweep: inner start + first direction, loop bodies, x += d, 3 certification kernels
-      launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * iterations_per_body(c) * body[0] + 1 + 3;
-      if (body[1]) { capped_by_bound = true; break; }
-    }
-  } else {
-    for (;;) {
-      if ((e = cudaGraphLaunch(c->graphs->attempt, s)) != cudaSuccess) return set_cuda_error(e);
-      if ((e = read_state(true)) != cudaSuccess) return set_cuda_error(e);
-      if (c->prec == PGJ_FP32)  // rel start + first direction, bodies, 3 per replacement, fold + certify
-        launches += 1 + first_direction_launches(c) + (c->four ? 5LL : 9LL) * iterations_per_body(c) * body[0] + 3LL * body[3] + 1 + 3;
-      else  // attempt: init mask + first direction, loop bodies, 3 certification kernels
-        launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * iterations_per_body(c) * body[0] + 3;
-      if (body[1]) { capped_by_bound = true; break; }
-      bool all, anybad, capped;
-      evaluate(all, anybad, capped);
-      if (all || restarts >= 2 || anybad || capped) break;
-      ++restarts;
-    }
+  // one FP32 inner solve per sweep inside FP64 iterative refinement
+  if ((e = read_state(false)) != cudaSuccess) return set_cuda_error(e);
+  for (;;) {
+    bool all, anybad, capped;
+    evaluate(all, anybad, capped);
+    if (all || anybad || capped || sweeps >= kMaxSweeps) break;
+    if ((e = cudaGraphLaunch(c->graphs->attempt, s)) != cudaSuccess) return set_cuda_error(e);
+    ++sweeps;
+    if ((e = read_state(true)) != cudaSuccess) return set_cuda_error(e);
+    // sweep: inner start + first direction, loop bodies, x += d, 3 certification kernels
+    launches += 1 + first_direction_launches(c) + (c->four ? 4LL : 8LL) * iterations_per_body(c) * body[0] + 1 + 3;
+    if (body[1]) { capped_by_bound = true; break; }
   }
   if (u != c->x) e = cudaMemcpyAsync(u, c->x, sizeof(double) * N3 * loads, cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -770,13 +753,13 @@ int pgj_solve(pgj_ctx* c, int loads, const double* macros, double rtol, double* 
     I.absolute_residual = h[l].absolute;
     I.threshold = thr;
     I.relative_residual = h[l].absolute / (h[l].norm > 1e-300 ? h[l].norm : 1e-300);
-    I.iterations = mixed ? h[l].total_iterations : h[l].iterations;
+    I.iterations = h[l].total_iterations;
     I.converged = ok[l];
-    I.restarts = restarts;
+    I.restarts = 0;
     I.bad = h[l].bad;
     all = all && ok[l];
   }
-  c->last_refinements = mixed ? sweeps : (c->prec == PGJ_FP32 ? 1 + body[3] : 1);
+  c->last_refinements = sweeps;
   c->last_launches = launches;
   if (body[2]) return PGJ_ERR_TIMEOUT;
   if (capped_by_bound) return PGJ_ERR_ITERATION_CAP;
@@ -920,8 +903,7 @@ int pgj_energies(pgj_ctx* c, int loads, const double* u, const double* macros, d
 
 int pgj_effective_tensor_at(pgj_ctx* c, int design, const double* u, double* C, void* stream) {
   if (!c || !u || !C || design < 0 || design >= c->D) return PGJ_ERR_ARGUMENT;
-  return launch_effective_tensor(c, c->a + size_t(design) * size_t(c->N), u, C, nullptr,
-                                 static_cast<cudaStream_t>(stream));
+  return launch_effective_tensor(c, c->a + size_t(design) * size_t(c->N), u, C, static_cast<cudaStream_t>(stream));
 }
 
 int pgj_effective_tensor(pgj_ctx* c, const double* u, double* C, void* stream) {

@@ -16,8 +16,8 @@ struct EnergyArgs {
   const double* u;       // (loads, 3N)
   const double* macros;  // (loads, 6) device
   const double* a;       // (N)
-  double* e;             // (loads, N) or null
-  double* C;             // 36 or null (pairs mode)
+  double* e;             // (loads, N): energies
+  double* C;             // 36: tensor
   LoadScalars* scal;     // ticket owner (record 0)
   double* partials;      // 21 * kMaxPartials
   OpConst kc;            // a = 1 constants of C0
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energies(const EnergyArgs A)
   }
 }
 
-// Tensor (and the energies, if asked for) of six loads: warp j owns load j. It publishes its modes, double-buffered
+// Tensor of six loads: warp j owns load j. It publishes its modes, double-buffered
 // over one barrier a step, and takes the pairs (j, j + k mod 6), k = 0, 1, 2, the first three warps also k = 3: each
 // of the 21 pairs once, so that the warps' work differs by one pair. Two blocks per SM: 158 registers; with three
 // the compiler has 96 and spills.
@@ -138,9 +138,7 @@ __global__ void __launch_bounds__(6 * kEnergyLanes, 2) k_tensor(const EnergyArgs
 #pragma unroll
       for (int c = 0; c < 3; ++c) buf[j * kLoad + ((m - 1) * 3 + c) * kEnergyLanes] = Q[m][c];
     element_modal<double>(Q, 1.0, A.kc, P);
-    const double own = energy_dot(Q, P);
-    acc[0] += ae * own;
-    if (A.e && i0 < nn) A.e[size_t(j) * N + size_t(z) * nn + i] = own * invv;
+    acc[0] += ae * energy_dot(Q, P);
     __syncthreads();  // modes published; the other parity's have been read
 #pragma unroll
     for (int k = 1; k < 4; ++k) {
@@ -223,11 +221,10 @@ int launch_energies(pgj_ctx* c, int loads, const double* u, const double* macros
   return check_launch();
 }
 
-int launch_effective_tensor(pgj_ctx* c, const double* a, const double* u, double* C, double* e, cudaStream_t s) {
+int launch_effective_tensor(pgj_ctx* c, const double* a, const double* u, double* C, cudaStream_t s) {
   EnergyArgs A = energy_args(c, 6, u, c->aux + kAuxVoigt);  // unit Voigt macros (6 x 6)
   A.a = a;
   A.C = C;
-  A.e = e;
   return launch_tensor(A, s);
 }
 

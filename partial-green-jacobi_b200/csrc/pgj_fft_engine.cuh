@@ -1,9 +1,5 @@
 // Shared-memory Stockham FFT engine (radices 2, 3, 4, 5, 8) used by the Green passes.
-//
-// Two forms of one stage: `stage` runs the butterflies of the single line a thread owns (threads
-// along y split them); `stage_lines` spreads the butterflies of many lines over a flat thread
-// range, line index fastest (lines at unit offset, e.g. columns) or butterfly index fastest
-// (contiguous rows), so shared-memory accesses of a warp stay on distinct banks.
+// `stage` runs the butterflies of the single line a thread owns (threads along y split them).
 #pragma once
 #include "pgj_internal.h"
 

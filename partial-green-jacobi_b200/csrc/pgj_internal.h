@@ -239,7 +239,7 @@ int launch_rel_fold(pgj_ctx* c, int loads, bool all, cudaStream_t s);
 int launch_rel_sync(pgj_ctx* c, int loads, cudaStream_t s);
 // energy (pgj_energy.cu)
 int launch_energies(pgj_ctx* c, int loads, const double* u, const double* macros_dev, double* e, cudaStream_t s);
-int launch_effective_tensor(pgj_ctx* c, const double* a, const double* u, double* C, double* e, cudaStream_t s);
+int launch_effective_tensor(pgj_ctx* c, const double* a, const double* u, double* C, cudaStream_t s);
 
 // Points the context's per-design views (a, scale) at design d for the lifetime of the scope, so that the
 // single-design scale build runs on it.
