@@ -173,7 +173,8 @@ int pgj_set_flexible_beta(pgj_ctx* ctx, int on);
  * apply and the vectors stay FP32. PGJ_FP64 contexts accept 1 only. */
 int pgj_set_mixed_operator(pgj_ctx* ctx, int fp64);
 /* Refinement count of the last pgj_solve: 1 for PGJ_FP64; sweeps in mixed mode 1; 1 + true-residual
- * replacements in mixed mode 0. */
+ * replacements in mixed mode 0 (iterations at which some load's residual was replaced; on grids of the
+ * resident kernel, the replacements of the load with most). */
 int pgj_last_refinements(pgj_ctx* ctx);
 
 /* Kernel launches issued by the last pgj_solve (graph nodes included), for launch accounting. */

@@ -88,7 +88,7 @@ __global__ void k_grid_wait_selftest(GridBar* bar, double* bounds, unsigned long
 // thread, kConeTaps taps at a time. Instructions bound it on large grids (tests, addresses and selects of a tap are
 // shared by a thread's cells), the latency of a group's loads on small ones. us a call, one cell per thread with a branch
 // per tap / four cells one after the other / this loop: 389 taps n = 24 54 / 217 / 35, 64 123 / 281 / 103, 128 647 /
-// 1403 / 543; 4169 taps n = 24 539 / 2235 / 330, 64 1165 / 2710 / 1026.
+// 1403 / 543; 4139 taps n = 24 539 / 2235 / 330, 64 1165 / 2710 / 1026.
 constexpr int kConeX = 32, kConeY = 8, kConeZ = 4, kConeR = 3, kConeTaps = 384;
 struct alignas(16) ConeTap {
   double w;
